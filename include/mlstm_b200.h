@@ -91,6 +91,14 @@ int mlstm_mm_bwd(const void* dh, const void* q, const void* k, const void* v, co
                  void* workspace, size_t workspace_bytes, int B, int NH, int S, int D, int dtype, int h_dtype,
                  int flags, void* stream);
 
+/* The same backward behind the output gate: dh is the gradient of h * silu(o), h the ungated result.  o and its
+ * gradient d_o [B,NH,S,D] of `dtype`; the gate's own derivative is taken in the pass that prepares the row vectors. */
+size_t mlstm_mm_bwd_ogate_workspace(int B, int NH, int S, int D, int dtype, int h_dtype, int flags);
+int mlstm_mm_bwd_ogate(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i,
+                       const void* h, const float* m, const float* b, const void* o, void* dq, void* dk, void* dv, void* df,
+                       void* di, void* d_o, void* workspace, size_t workspace_bytes, int B, int NH, int S, int D, int dtype,
+                       int h_dtype, int flags, void* stream);
+
 /* Forward scan with output gate: h = mLSTM(q, k, v, f, i) * silu(o).
  * Replaces the four launches of mlstm_scan (mlstm_scan.py:281-327): stabilize_fi (:47-69),
  * precompute_mlstm_triton_scan (:74-137), reduce_mlstm_triton (:143-195), mlstm_triton_scan
@@ -190,7 +198,8 @@ int mlstm_chunk_apply(const void* q, const void* k, const void* v, const void* o
  *                         of the workspace (what the parallel forward returns as M and B)
  *   mlstm_chunk_bwd       dh, h of `h_dtype` (fp32 or the input type); q, k, v, f, i and dq, dk, dv, df, di of
  *                         `dtype`; m, b as read above.  Its workspace is its own (mlstm_chunk_bwd_workspace);
- *                         the gates and block states are recomputed in it.  df[..., 0] is exactly 0. */
+ *                         the gates and block states are recomputed in it.  df[..., 0] is exactly 0.
+ *   mlstm_chunk_bwd_ogate the same behind the output gate, see mlstm_mm_bwd_ogate */
 int mlstm_chunk_read_mb(const void* workspace, size_t workspace_bytes, float* m, float* b, int B, int NH, int S, int D,
                         int dtype, int chunk, void* stream);
 size_t mlstm_chunk_bwd_workspace(int B, int NH, int S, int D, int dtype, int h_dtype, int chunk);
@@ -198,6 +207,11 @@ int mlstm_chunk_bwd(const void* dh, const void* q, const void* k, const void* v,
                     const void* h, const float* m, const float* b, void* dq, void* dk, void* dv, void* df, void* di,
                     void* workspace, size_t workspace_bytes, int B, int NH, int S, int D, int dtype, int h_dtype,
                     int chunk, void* stream);
+size_t mlstm_chunk_bwd_ogate_workspace(int B, int NH, int S, int D, int dtype, int h_dtype, int chunk);
+int mlstm_chunk_bwd_ogate(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i,
+                          const void* h, const float* m, const float* b, const void* o, void* dq, void* dk, void* dv,
+                          void* df, void* di, void* d_o, void* workspace, size_t workspace_bytes, int B, int NH, int S,
+                          int D, int dtype, int h_dtype, int chunk, void* stream);
 
 /* Sequence-parallel form of the chunkwise forward: rank r of `world` holds the r-th contiguous segment
  * of every sequence, and ONE exchange connects the ranks (the carry combine of mlstm_scan.py:15-26

@@ -54,6 +54,10 @@ def lib():
     L.mlstm_mm_bwd_workspace.argtypes = [i32] * 7
     L.mlstm_mm_bwd.restype = i32
     L.mlstm_mm_bwd.argtypes = [vp] * 14 + [vp, sz] + [i32] * 7 + [vp]
+    L.mlstm_mm_bwd_ogate_workspace.restype = sz
+    L.mlstm_mm_bwd_ogate_workspace.argtypes = [i32] * 7
+    L.mlstm_mm_bwd_ogate.restype = i32
+    L.mlstm_mm_bwd_ogate.argtypes = [vp] * 16 + [vp, sz] + [i32] * 7 + [vp]
     L.mlstm_scan_fwd_workspace.restype = sz
     L.mlstm_scan_fwd_workspace.argtypes = [i32] * 6
     L.mlstm_scan_fwd.restype = i32
@@ -90,6 +94,10 @@ def lib():
     L.mlstm_chunk_bwd_workspace.argtypes = [i32] * 7
     L.mlstm_chunk_bwd.restype = i32
     L.mlstm_chunk_bwd.argtypes = [vp] * 14 + [vp, sz] + [i32] * 7 + [vp]
+    L.mlstm_chunk_bwd_ogate_workspace.restype = sz
+    L.mlstm_chunk_bwd_ogate_workspace.argtypes = [i32] * 7
+    L.mlstm_chunk_bwd_ogate.restype = i32
+    L.mlstm_chunk_bwd_ogate.argtypes = [vp] * 16 + [vp, sz] + [i32] * 7 + [vp]
     L.mlstm_forward_f16_static_status.restype = i32
     L.mlstm_forward_f16_static_status.argtypes = [ctypes.POINTER(i32), vp]
     L.mlstm_ogate_fwd.restype = i32
@@ -106,7 +114,8 @@ def lib():
 
 EXPORTS = [
     "mlstm_status_string", "mlstm_last_error_detail", "mlstm_tc_supported", "mlstm_mm_fwd_workspace", "mlstm_mm_fwd",
-    "mlstm_mm_bwd_workspace", "mlstm_mm_bwd", "mlstm_scan_fwd_workspace", "mlstm_scan_fwd",
+    "mlstm_mm_bwd_workspace", "mlstm_mm_bwd", "mlstm_mm_bwd_ogate_workspace", "mlstm_mm_bwd_ogate",
+    "mlstm_chunk_bwd_ogate_workspace", "mlstm_chunk_bwd_ogate", "mlstm_scan_fwd_workspace", "mlstm_scan_fwd",
     "mlstm_forward_f16_workspace", "mlstm_forward_f16", "mlstm_forward_f16_static", "mlstm_backward_f16_workspace",
     "mlstm_backward_f16", "mlstm_read_status",
     "mlstm_chunk_workspace", "mlstm_chunk_gate_summary", "mlstm_chunk_prepare", "mlstm_chunk_local_state",

@@ -80,7 +80,8 @@ struct BwdWs {
     void* dh16;
     size_t bytes;
 };
-BwdWs carve_bwd(void* ws, int BH, int S, int D, bool need_dh16) {
+// dh_copy_es: bytes per element of a copy of dh (in the inputs' type, or taken through the output gate); 0: none
+BwdWs carve_bwd(void* ws, int BH, int S, int D, int dh_copy_es) {
     Carver c(ws);
     BwdWs w{};
     const size_t vec = static_cast<size_t>(BH) * round_up(S, TILE) * sizeof(float);
@@ -95,7 +96,7 @@ BwdWs carve_bwd(void* ws, int BH, int S, int D, bool need_dh16) {
     w.g = c.take<float>(vec);
     w.dI = c.take<float>(vec * TC_DOT_PARTS);   // partial row dots, one per gate group of the tensor-core passes
     w.R = c.take<float>(vec * TC_DOT_PARTS);
-    w.dh16 = need_dh16 ? c.take<uint8_t>(static_cast<size_t>(BH) * S * D * 2) : nullptr;
+    w.dh16 = dh_copy_es ? c.take<uint8_t>(static_cast<size_t>(BH) * S * D * dh_copy_es) : nullptr;
     w.bytes = c.off;
     return w;
 }
@@ -304,18 +305,32 @@ int mlstm_mm_fwd(const void* q, const void* k, const void* v, const void* f, con
                         static_cast<cudaStream_t>(stream), extra ? static_cast<uint8_t*>(workspace) + w.bytes : nullptr);
 }
 
-size_t mlstm_mm_bwd_workspace(int B, int NH, int S, int D, int dtype, int h_dtype, int flags) {
-    if (check_dims(B, NH, S, D) != MLSTM_OK) return 0;
-    if (mm_bwd_two_pass(S, D, dtype, flags))
-        return carve_bwd(nullptr, B * NH, S, D, dtype != MLSTM_DT_F32 && h_dtype != dtype).bytes +
-               two_pass_bwd_extra_bytes(B * NH, S, D, dtype);
-    return carve_bwd(nullptr, B * NH, S, D, dtype != MLSTM_DT_F32 && h_dtype != dtype).bytes +
-           tf32_copy_bytes(B * NH, S, D, dtype, flags, 4);
+// The passes read dh in the inputs' type: a copy where h (and with it dh) has another one, or where dh is first taken
+// through the output gate.
+static int dh_copy_bytes(int dtype, int h_dtype, bool gated) {
+    if (dtype == MLSTM_DT_F32) return gated ? 4 : 0;
+    return (gated || h_dtype != dtype) ? 2 : 0;
 }
 
-int mlstm_mm_bwd(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h,
-                 const float* m, const float* b, void* dq, void* dk, void* dv, void* df, void* di, void* workspace,
-                 size_t workspace_bytes, int B, int NH, int S, int D, int dtype, int h_dtype, int flags, void* stream) {
+static size_t mm_bwd_workspace(int B, int NH, int S, int D, int dtype, int h_dtype, int flags, bool gated) {
+    if (check_dims(B, NH, S, D) != MLSTM_OK) return 0;
+    const size_t own = carve_bwd(nullptr, B * NH, S, D, dh_copy_bytes(dtype, h_dtype, gated)).bytes;
+    if (mm_bwd_two_pass(S, D, dtype, flags)) return own + two_pass_bwd_extra_bytes(B * NH, S, D, dtype);
+    return own + tf32_copy_bytes(B * NH, S, D, dtype, flags, 4);
+}
+
+size_t mlstm_mm_bwd_workspace(int B, int NH, int S, int D, int dtype, int h_dtype, int flags) {
+    return mm_bwd_workspace(B, NH, S, D, dtype, h_dtype, flags, false);
+}
+
+size_t mlstm_mm_bwd_ogate_workspace(int B, int NH, int S, int D, int dtype, int h_dtype, int flags) {
+    return mm_bwd_workspace(B, NH, S, D, dtype, h_dtype, flags, true);
+}
+
+static int mm_bwd_impl(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h,
+                       const float* m, const float* b, const void* o, void* d_o, void* dq, void* dk, void* dv, void* df, void* di,
+                       void* workspace, size_t workspace_bytes, int B, int NH, int S, int D, int dtype, int h_dtype, int flags,
+                       void* stream) {
     if (!dh || !q || !k || !v || !f || !i || !h || !m || !b || !dq || !dk || !dv || !df || !di) return MLSTM_E_ARG;
     if (!dtype_ok(dtype) || (h_dtype != MLSTM_DT_F32 && h_dtype != dtype)) return MLSTM_E_ARG;
     int rc = check_dims(B, NH, S, D);
@@ -324,8 +339,8 @@ int mlstm_mm_bwd(const void* dh, const void* q, const void* k, const void* v, co
         !aligned16(dk) || !aligned16(dv))
         return MLSTM_E_ALIGN;
     const int BH = B * NH, Spad = round_up(S, TILE);
-    const bool need16 = dtype != MLSTM_DT_F32 && h_dtype != dtype;
-    BwdWs w = carve_bwd(workspace, BH, S, D, need16);
+    const int dh_es = dh_copy_bytes(dtype, h_dtype, o != nullptr);
+    BwdWs w = carve_bwd(workspace, BH, S, D, dh_es);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (mm_bwd_two_pass(S, D, dtype, flags)) {
         if (!workspace || workspace_bytes < w.bytes + two_pass_bwd_extra_bytes(BH, S, D, dtype) || !aligned16(workspace))
@@ -334,14 +349,14 @@ int mlstm_mm_bwd(const void* dh, const void* q, const void* k, const void* v, co
         if ((rc = launch_gates_fwd(f, i, w.ga, w.gAn, w.a_ref, w.An_ref, nullptr, BH, S, Spad, dtype, st, nullptr, nullptr, nullptr,
                                    0, nullptr, w.gaw, w.status, STATUS_WORDS)) != MLSTM_OK)
             return rc;
-        if ((rc = launch_bwd_prep(h, dh, b, m, w.gAn, w.gB, w.gBw, w.g, w.dh16, BH, S, Spad, D, h_dtype, dtype, st)) != MLSTM_OK)
+        if ((rc = launch_bwd_prep(h, dh, b, m, w.gAn, w.gB, w.gBw, w.g, w.dh16, o, d_o, BH, S, Spad, D, h_dtype, dtype, st)) != MLSTM_OK)
             return rc;
         const size_t vec = static_cast<size_t>(BH) * Spad * sizeof(float);
         const size_t mat = al(scan_gemm_bwd_matrix_bytes(BH, S, dtype));
         uint8_t* extra_base = static_cast<uint8_t*>(workspace) + w.bytes;
         ScanGemmBwdArgs a{};
         a.S = S; a.Spad = Spad; a.BH = BH; a.D = D;
-        a.q = q; a.k = k; a.v = v; a.dh = need16 ? w.dh16 : dh;
+        a.q = q; a.k = k; a.v = v; a.dh = dh_es ? w.dh16 : dh;
         a.dq = dq; a.dk = dk; a.dv = dv;
         a.ga = w.ga; a.gaw = w.gaw; a.gB = w.gB; a.g = w.g; a.a_ref = w.a_ref; a.An_ref = w.An_ref;
         a.Wn = extra_base; a.dT = extra_base + mat;
@@ -360,9 +375,9 @@ int mlstm_mm_bwd(const void* dh, const void* q, const void* k, const void* v, co
     if ((rc = launch_gates_fwd(f, i, w.ga, w.gAn, w.a_ref, w.An_ref, nullptr, BH, S, Spad, dtype, st, nullptr, nullptr, nullptr, 0,
                                nullptr, w.gaw, w.status, STATUS_WORDS)) != MLSTM_OK)
         return rc;
-    if ((rc = launch_bwd_prep(h, dh, b, m, w.gAn, w.gB, w.gBw, w.g, w.dh16, BH, S, Spad, D, h_dtype, dtype, st)) != MLSTM_OK)
+    if ((rc = launch_bwd_prep(h, dh, b, m, w.gAn, w.gB, w.gBw, w.g, w.dh16, o, d_o, BH, S, Spad, D, h_dtype, dtype, st)) != MLSTM_OK)
         return rc;
-    const void* dhp = need16 ? w.dh16 : dh;  // dh in the element type of q, k, v
+    const void* dhp = dh_es ? w.dh16 : dh;  // dh in the element type of q, k, v
     const void* orig_q = q;
     const void* orig_k = k;
     if (kind != KIND_SIMT && dtype == MLSTM_DT_F32) {  // converted copies of q, k, v, dh
@@ -392,6 +407,23 @@ int mlstm_mm_bwd(const void* dh, const void* q, const void* k, const void* v, co
     if ((rc = run_pass(kind, DV, p, dtype, dtype, st)) != MLSTM_OK) return rc;
     return launch_df(f, w.dI, w.R, df, di, BH, S, Spad, dtype, st, kind == KIND_SIMT ? 1 : TC_DOT_PARTS,
                      static_cast<long long>(BH) * Spad);
+}
+
+int mlstm_mm_bwd(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h,
+                 const float* m, const float* b, void* dq, void* dk, void* dv, void* df, void* di, void* workspace,
+                 size_t workspace_bytes, int B, int NH, int S, int D, int dtype, int h_dtype, int flags, void* stream) {
+    return mm_bwd_impl(dh, q, k, v, f, i, h, m, b, nullptr, nullptr, dq, dk, dv, df, di, workspace, workspace_bytes, B, NH, S, D,
+                       dtype, h_dtype, flags, stream);
+}
+
+int mlstm_mm_bwd_ogate(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h,
+                       const float* m, const float* b, const void* o, void* dq, void* dk, void* dv, void* df, void* di, void* d_o,
+                       void* workspace, size_t workspace_bytes, int B, int NH, int S, int D, int dtype, int h_dtype, int flags,
+                       void* stream) {
+    if (!o || !d_o) return MLSTM_E_ARG;
+    if (!aligned16(o) || !aligned16(d_o)) return MLSTM_E_ALIGN;
+    return mm_bwd_impl(dh, q, k, v, f, i, h, m, b, o, d_o, dq, dk, dv, df, di, workspace, workspace_bytes, B, NH, S, D, dtype,
+                       h_dtype, flags, stream);
 }
 
 // Which of its three forms the scan entry uses.

@@ -498,9 +498,15 @@ size_t mlstm_chunk_bwd_workspace(int B, int NH, int S, int D, int dtype, int h_d
     return carve_bwd_chunk(nullptr, B * NH, S, D, chunk, h_dtype != dtype).bytes;
 }
 
-int mlstm_chunk_bwd(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h,
-                    const float* m, const float* b, void* dq, void* dk, void* dv, void* df, void* di, void* workspace,
-                    size_t workspace_bytes, int B, int NH, int S, int D, int dtype, int h_dtype, int chunk, void* stream) {
+size_t mlstm_chunk_bwd_ogate_workspace(int B, int NH, int S, int D, int dtype, int h_dtype, int chunk) {
+    if (check_chunk_args(B, NH, S, D, dtype, chunk) != MLSTM_OK) return 0;
+    return carve_bwd_chunk(nullptr, B * NH, S, D, chunk, true).bytes;
+}
+
+static int chunk_bwd_impl(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h,
+                          const float* m, const float* b, const void* o, void* d_o, void* dq, void* dk, void* dv, void* df, void* di,
+                          void* workspace, size_t workspace_bytes, int B, int NH, int S, int D, int dtype, int h_dtype, int chunk,
+                          void* stream) {
     if (!dh || !q || !k || !v || !f || !i || !h || !m || !b || !dq || !dk || !dv || !df || !di) return MLSTM_E_ARG;
     int rc = check_chunk_args(B, NH, S, D, dtype, chunk);
     if (rc != MLSTM_OK) return rc;
@@ -509,7 +515,7 @@ int mlstm_chunk_bwd(const void* dh, const void* q, const void* k, const void* v,
         !aligned16(dk) || !aligned16(dv))
         return MLSTM_E_ALIGN;
     const int BH = B * NH, Spad = round_up(S, TILE);
-    const bool need16 = h_dtype != dtype;
+    const bool need16 = o || h_dtype != dtype;   // dh in the input type, taken through the output gate where there is one
     ChunkBwdWs w = carve_bwd_chunk(workspace, BH, S, D, chunk, need16);
     if (!workspace || workspace_bytes < w.bytes || !aligned16(workspace)) return MLSTM_E_WORKSPACE;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -532,7 +538,7 @@ int mlstm_chunk_bwd(const void* dh, const void* q, const void* k, const void* v,
                                 dtype, st, nullptr, nullptr, 0, nullptr, w.statesT, 0)) != MLSTM_OK)
         return rc;
     // delta = dh . h, n, db -> the backward's per-row vectors (and dh in the input type)
-    if ((rc = launch_bwd_prep(h, dh, b, m, c.gAn, w.gB, w.gBw, w.g, w.dh16, BH, S, Spad, D, h_dtype, dtype, st)) != MLSTM_OK)
+    if ((rc = launch_bwd_prep(h, dh, b, m, c.gAn, w.gB, w.gBw, w.g, w.dh16, o, d_o, BH, S, Spad, D, h_dtype, dtype, st)) != MLSTM_OK)
         return rc;
     const void* dhp = need16 ? w.dh16 : dh;
     // what every block contributes to the state carried back: P_k = sum_t beta_t q_t dh_t^T (tensor cores), p_k (vector)
@@ -575,6 +581,23 @@ int mlstm_chunk_bwd(const void* dh, const void* q, const void* k, const void* v,
     p.out = dv; p.dot_src = nullptr; p.dot_out = nullptr;
     if ((rc = launch_pass_tc(DVC, p, dtype, dtype, st)) != MLSTM_OK) return rc;
     return launch_df(f, w.dI, w.Rdot, df, di, BH, S, Spad, dtype, st, TC_DOT_PARTS, static_cast<long long>(BH) * Spad, c.gscratch);
+}
+
+int mlstm_chunk_bwd(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h,
+                    const float* m, const float* b, void* dq, void* dk, void* dv, void* df, void* di, void* workspace,
+                    size_t workspace_bytes, int B, int NH, int S, int D, int dtype, int h_dtype, int chunk, void* stream) {
+    return chunk_bwd_impl(dh, q, k, v, f, i, h, m, b, nullptr, nullptr, dq, dk, dv, df, di, workspace, workspace_bytes, B, NH, S, D,
+                          dtype, h_dtype, chunk, stream);
+}
+
+int mlstm_chunk_bwd_ogate(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h,
+                          const float* m, const float* b, const void* o, void* dq, void* dk, void* dv, void* df, void* di, void* d_o,
+                          void* workspace, size_t workspace_bytes, int B, int NH, int S, int D, int dtype, int h_dtype, int chunk,
+                          void* stream) {
+    if (!o || !d_o) return MLSTM_E_ARG;
+    if (!aligned16(o) || !aligned16(d_o)) return MLSTM_E_ALIGN;
+    return chunk_bwd_impl(dh, q, k, v, f, i, h, m, b, o, d_o, dq, dk, dv, df, di, workspace, workspace_bytes, B, NH, S, D, dtype,
+                          h_dtype, chunk, stream);
 }
 
 int mlstm_chunk_read_mb(const void* workspace, size_t workspace_bytes, float* m, float* b, int B, int NH, int S, int D, int dtype,

@@ -267,24 +267,37 @@ __global__ void gates_fold_kernel(const double* __restrict__ local, const double
     }
 }
 
-// One warp per row: delta = dh.h, n, db, and from them the two per-row vectors of the backward:
+// One warp per PREP_ROWS rows: delta = dh.h, n, db, and from them the two per-row vectors of the backward:
 //   gB_rel = gAn_rel + log2(scale / n)  (same block references as gAn_rel),   g = db * n
 // (db = sign(b) * (-delta / n) * [|b| > exp(-m)], mlstm_matmul.py:194-196 with the sum replaced by
-// n*delta).  Optionally writes dh converted to the 16-bit input type for the tensor-core passes.
+// n*delta).  Optionally writes dh converted to the inputs' type for the contraction passes.
+// GATED: the output was h * silu(o).  dh is then the gradient of the gated output: it is taken through the gate here,
+// dh_inner = dh silu(o) (to dh_out) and d_o = dh h silu'(o) with silu'(x) = sigma(x) (1 + x (1 - sigma(x))), so that the
+// gate's backward costs no pass of its own.  Bound by HBM: dh, h, o in, dh_out, d_o out, 14 bytes per element (16-bit
+// inputs, fp32 h) where the gate's own kernel and this one moved 26.
 // Rows are read with 16-byte accesses.  Padding rows: gB_rel = -inf, g = 0.
 constexpr int PREP_ROWS = 4;   // positions per warp in bwd_prep_kernel
 
-template <typename HT, typename T16>
+// V consecutive values as one access
+template <typename T, int V>
+struct alignas(sizeof(T) * V) VecOf {
+    T v[V];
+};
+
+template <typename HT, typename T16, bool GATED>
 __global__ void bwd_prep_kernel(const HT* __restrict__ h, const HT* __restrict__ dh, const float* __restrict__ b,
                                 const float* __restrict__ m, const float* __restrict__ gAn_rel,
                                 float* __restrict__ gB_rel, float* __restrict__ gB_w, float* __restrict__ g,
-                                T16* __restrict__ dh16, int BH, int S, int Spad, int D, float log2_scale) {
+                                T16* __restrict__ dh_out, const T16* __restrict__ o, T16* __restrict__ d_o, int BH, int S,
+                                int Spad, int D, float log2_scale) {
     grid_dep_wait();
     grid_dep_launch();
     // A warp takes PREP_ROWS consecutive positions of one slice (Spad is a multiple of 128): all of their row
     // loads and the per-position scalars are requested before anything is used, so a warp pays the memory
     // latency once instead of twice per position.
     constexpr int VEC = 16 / sizeof(HT);
+    using VH = VecOf<HT, VEC>;
+    using VT = VecOf<T16, VEC>;
     const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const long long first = static_cast<long long>(warp_global) * PREP_ROWS;
@@ -303,21 +316,41 @@ __global__ void bwd_prep_kernel(const HT* __restrict__ h, const HT* __restrict__
     }
     float delta[PREP_ROWS];
 #pragma unroll
-    for (int r = 0; r < PREP_ROWS; r++) {
-        delta[r] = 0.0f;
-        if (t0 + r < S) {
-            const size_t row = (static_cast<size_t>(bh) * S + t0 + r) * D;
-            for (int d = lane * VEC; d < D; d += 32 * VEC) {
-                const uint4 hraw = *reinterpret_cast<const uint4*>(h + row + d);
-                const uint4 draw = *reinterpret_cast<const uint4*>(dh + row + d);
-                const HT* hv = reinterpret_cast<const HT*>(&hraw);
-                const HT* dv = reinterpret_cast<const HT*>(&draw);
+    for (int r = 0; r < PREP_ROWS; r++) delta[r] = 0.0f;
+    const size_t row0 = (static_cast<size_t>(bh) * S + t0) * D;
+    for (int d = lane * VEC; d < D; d += 32 * VEC) {
+        VH hv[PREP_ROWS], dv[PREP_ROWS];
+        [[maybe_unused]] VT ov[PREP_ROWS];
+#pragma unroll
+        for (int r = 0; r < PREP_ROWS; r++) {
+            if (t0 + r < S) {
+                const size_t at = row0 + static_cast<size_t>(r) * D + d;
+                hv[r] = *reinterpret_cast<const VH*>(h + at);
+                dv[r] = *reinterpret_cast<const VH*>(dh + at);
+                if constexpr (GATED) ov[r] = *reinterpret_cast<const VT*>(o + at);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < PREP_ROWS; r++) {
+            if (t0 + r < S) {
+                const size_t at = row0 + static_cast<size_t>(r) * D + d;
+                VT out;
+                [[maybe_unused]] VT dov;
 #pragma unroll
                 for (int j = 0; j < VEC; j++) {
-                    const float x = to_f32<HT>(dv[j]);
-                    delta[r] += x * to_f32<HT>(hv[j]);
-                    if (dh16) dh16[row + d + j] = from_f32<T16>(x);
+                    float x = to_f32<HT>(dv[r].v[j]);
+                    const float hi = to_f32<HT>(hv[r].v[j]);
+                    if constexpr (GATED) {
+                        const float ox = to_f32<T16>(ov[r].v[j]);
+                        const float sg = 1.0f / (1.0f + __expf(-ox));
+                        dov.v[j] = from_f32<T16>(x * hi * sg * (1.0f + ox * (1.0f - sg)));
+                        x *= ox * sg;
+                    }
+                    delta[r] += x * hi;
+                    out.v[j] = from_f32<T16>(x);
                 }
+                if (dh_out) *reinterpret_cast<VT*>(dh_out + at) = out;
+                if constexpr (GATED) *reinterpret_cast<VT*>(d_o + at) = dov;
             }
         }
     }
@@ -326,7 +359,7 @@ __global__ void bwd_prep_kernel(const HT* __restrict__ h, const HT* __restrict__
     for (int r = 0; r < PREP_ROWS; r++) {
         float x = delta[r];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        for (int o2 = 16; o2 > 0; o2 >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o2);
         if (lane == r) my_delta = x;
     }
     if (mine) {
@@ -430,27 +463,52 @@ __global__ void __launch_bounds__(SCAN_THREADS) df_kernel(const T* __restrict__ 
 
 // Output gate, elementwise: h = h_inner * silu(o) (mlstm_scan.py:273-278; the "integrate o" note at
 // mlstm_matmul.py:36) and its derivative: dh_inner = dh * silu(o), do = dh * h_inner * silu'(o) with
-// silu'(x) = sigma(x) (1 + x (1 - sigma(x))).  Eight elements per thread, 16-byte accesses on the 16-bit side.
-template <typename HT, typename OT, bool BWD>
-__global__ void ogate_kernel(const HT* __restrict__ dh, const HT* __restrict__ h_inner, const OT* __restrict__ o,
-                             HT* __restrict__ out_h, OT* __restrict__ out_o, long long n) {
+// silu'(x) = sigma(x) (1 + x (1 - sigma(x))).
+// Bound by HBM.  A thread takes OGATE_U pieces of four values, 256 threads apart: a warp's accesses are contiguous (512
+// bytes of fp32, 256 of 16-bit values) and all of a thread's loads are in flight at once.  Eight consecutive values per
+// thread read one by one ran at 2.4 TB/s (0.57 ms for 1.35 GB).  VEC = 1: tensors that are not 16-byte aligned.
+constexpr int OGATE_THREADS = 256, OGATE_U = 4;
+template <typename HT, typename OT, bool BWD, int VEC>
+__global__ void __launch_bounds__(OGATE_THREADS) ogate_kernel(const HT* __restrict__ dh, const HT* __restrict__ h_inner,
+                                                              const OT* __restrict__ o, HT* __restrict__ out_h,
+                                                              OT* __restrict__ out_o, long long n) {
     grid_dep_wait();
     grid_dep_launch();
-    const long long base = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8;
-    if (base >= n) return;
+    using VH = VecOf<HT, VEC>;
+    using VO = VecOf<OT, VEC>;
+    const long long base = static_cast<long long>(blockIdx.x) * (OGATE_THREADS * OGATE_U * VEC) + threadIdx.x * VEC;
+    VH hv[OGATE_U], gv[OGATE_U];
+    VO ov[OGATE_U];
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const long long e = base + j;
-        if (e >= n) break;
-        const float x = to_f32<OT>(o[e]);
-        const float sg = 1.0f / (1.0f + __expf(-x));
-        const float hi = to_f32<HT>(h_inner[e]);
-        if (BWD) {
-            const float g = to_f32<HT>(dh[e]);
-            out_h[e] = from_f32<HT>(g * x * sg);
-            out_o[e] = from_f32<OT>(g * hi * sg * (1.0f + x * (1.0f - sg)));
-        } else {
-            out_h[e] = from_f32<HT>(hi * x * sg);
+    for (int u = 0; u < OGATE_U; u++) {
+        const long long e = base + static_cast<long long>(u) * OGATE_THREADS * VEC;
+        if (e < n) {       // (n is a multiple of VEC)
+            ov[u] = *reinterpret_cast<const VO*>(o + e);
+            hv[u] = *reinterpret_cast<const VH*>(h_inner + e);
+            if (BWD) gv[u] = *reinterpret_cast<const VH*>(dh + e);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < OGATE_U; u++) {
+        const long long e = base + static_cast<long long>(u) * OGATE_THREADS * VEC;
+        if (e < n) {
+            VH rh;
+            [[maybe_unused]] VO ro;
+#pragma unroll
+            for (int j = 0; j < VEC; j++) {
+                const float x = to_f32<OT>(ov[u].v[j]);
+                const float sg = 1.0f / (1.0f + __expf(-x));
+                const float hi = to_f32<HT>(hv[u].v[j]);
+                if (BWD) {
+                    const float g = to_f32<HT>(gv[u].v[j]);
+                    rh.v[j] = from_f32<HT>(g * x * sg);
+                    ro.v[j] = from_f32<OT>(g * hi * sg * (1.0f + x * (1.0f - sg)));
+                } else {
+                    rh.v[j] = from_f32<HT>(hi * x * sg);
+                }
+            }
+            *reinterpret_cast<VH*>(out_h + e) = rh;
+            if (BWD) *reinterpret_cast<VO*>(out_o + e) = ro;
         }
     }
 }
@@ -458,12 +516,20 @@ __global__ void ogate_kernel(const HT* __restrict__ dh, const HT* __restrict__ h
 template <bool BWD>
 static int ogate_dispatch(const void* dh, const void* h_inner, const void* o, void* out_h, void* out_o, long long n, int h_dtype,
                           int o_dtype, cudaStream_t st) {
-    const int threads = 256;
-    const long long blocks = (n + threads * 8 - 1) / (threads * 8);
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(dh) | reinterpret_cast<uintptr_t>(h_inner) | reinterpret_cast<uintptr_t>(o) |
+                           reinterpret_cast<uintptr_t>(out_h) | reinterpret_cast<uintptr_t>(out_o);
+    const bool vec4 = (bits & 15) == 0 && (n & 3) == 0;
+    const long long per_block = static_cast<long long>(OGATE_THREADS) * OGATE_U * (vec4 ? 4 : 1);
+    const long long blocks = (n + per_block - 1) / per_block;
     if (blocks <= 0 || blocks > 0x7fffffffLL) return MLSTM_E_SHAPE;
-#define OGATE_LAUNCH(HT, OT)                                                                                              \
-    ogate_kernel<HT, OT, BWD><<<(unsigned)blocks, threads, 0, st>>>((const HT*)dh, (const HT*)h_inner, (const OT*)o, (HT*)out_h, \
-                                                                    (OT*)out_o, n)
+#define OGATE_LAUNCH_V(HT, OT, V)                                                                                      \
+    ogate_kernel<HT, OT, BWD, V><<<(unsigned)blocks, OGATE_THREADS, 0, st>>>((const HT*)dh, (const HT*)h_inner, (const OT*)o, \
+                                                                             (HT*)out_h, (OT*)out_o, n)
+#define OGATE_LAUNCH(HT, OT)                        \
+    do {                                            \
+        if (vec4) OGATE_LAUNCH_V(HT, OT, 4);        \
+        else OGATE_LAUNCH_V(HT, OT, 1);             \
+    } while (0)
     if (h_dtype == MLSTM_DT_F32) {
         if (o_dtype == MLSTM_DT_F32) OGATE_LAUNCH(float, float);
         else if (o_dtype == MLSTM_DT_F16) OGATE_LAUNCH(float, __half);
@@ -477,6 +543,7 @@ static int ogate_dispatch(const void* dh, const void* h_inner, const void* o, vo
         return MLSTM_E_ARG;
     }
 #undef OGATE_LAUNCH
+#undef OGATE_LAUNCH_V
     return cudaGetLastError() == cudaSuccess ? MLSTM_OK : MLSTM_E_CUDA;
 }
 
@@ -653,31 +720,42 @@ int launch_gates_fwd(const void* f, const void* i, float* ga, float* gA, double*
     return MLSTM_E_ARG;
 }
 
-template <typename HT>
+template <typename HT, bool GATED>
 static int bwd_prep_dispatch(const void* h, const void* dh, const float* b, const float* m, const float* gA, float* gB,
-                             float* gBw, float* g, void* dh16, int BH, int S, int Spad, int D, int dtype, cudaStream_t st) {
+                             float* gBw, float* g, void* dh_out, const void* o, void* d_o, int BH, int S, int Spad, int D,
+                             int dtype, cudaStream_t st) {
     const long long warps = static_cast<long long>(BH) * Spad / PREP_ROWS;   // Spad is a multiple of 128
     const int threads = 256;
     const long long blocks = (warps * 32 + threads - 1) / threads;
     if (blocks > 0x7fffffffLL) return MLSTM_E_SHAPE;
     const float log2_scale = -0.5f * log2f(static_cast<float>(D));
+    const dim3 grid((unsigned)blocks), block(threads);
     if (dtype == MLSTM_DT_BF16)
-        launch_plain(bwd_prep_kernel<HT, __nv_bfloat16>, dim3((unsigned)blocks), dim3(threads), 0, st, 
-            (const HT*)h, (const HT*)dh, b, m, gA, gB, gBw, g, (__nv_bfloat16*)dh16, BH, S, Spad, D, log2_scale);
+        launch_plain(bwd_prep_kernel<HT, __nv_bfloat16, GATED>, grid, block, 0, st, (const HT*)h, (const HT*)dh, b, m, gA, gB, gBw, g,
+                     (__nv_bfloat16*)dh_out, (const __nv_bfloat16*)o, (__nv_bfloat16*)d_o, BH, S, Spad, D, log2_scale);
+    else if (dtype == MLSTM_DT_F16)
+        launch_plain(bwd_prep_kernel<HT, __half, GATED>, grid, block, 0, st, (const HT*)h, (const HT*)dh, b, m, gA, gB, gBw, g,
+                     (__half*)dh_out, (const __half*)o, (__half*)d_o, BH, S, Spad, D, log2_scale);
+    else if constexpr (sizeof(HT) == 4)
+        launch_plain(bwd_prep_kernel<HT, float, GATED>, grid, block, 0, st, (const HT*)h, (const HT*)dh, b, m, gA, gB, gBw, g,
+                     (float*)dh_out, (const float*)o, (float*)d_o, BH, S, Spad, D, log2_scale);
     else
-        launch_plain(bwd_prep_kernel<HT, __half>, dim3((unsigned)blocks), dim3(threads), 0, st, (const HT*)h, (const HT*)dh, b, m, gA, gB, gBw, g,
-                                                                         (__half*)dh16, BH, S, Spad, D, log2_scale);
+        return MLSTM_E_ARG;
     return cudaGetLastError() == cudaSuccess ? MLSTM_OK : MLSTM_E_CUDA;
 }
 
 int launch_bwd_prep(const void* h, const void* dh, const float* b, const float* m, const float* gA, float* gB, float* gBw,
-                    float* g, void* dh16, int BH, int S, int Spad, int D, int h_dtype, int dtype, cudaStream_t st) {
+                    float* g, void* dh_out, const void* o, void* d_o, int BH, int S, int Spad, int D, int h_dtype, int dtype,
+                    cudaStream_t st) {
+#define PREP(HT)                                                                                                          \
+    return o ? bwd_prep_dispatch<HT, true>(h, dh, b, m, gA, gB, gBw, g, dh_out, o, d_o, BH, S, Spad, D, dtype, st)         \
+             : bwd_prep_dispatch<HT, false>(h, dh, b, m, gA, gB, gBw, g, dh_out, nullptr, nullptr, BH, S, Spad, D, dtype, st)
     switch (h_dtype) {
-        case MLSTM_DT_F32: return bwd_prep_dispatch<float>(h, dh, b, m, gA, gB, gBw, g, dh16, BH, S, Spad, D, dtype, st);
-        case MLSTM_DT_F16: return bwd_prep_dispatch<__half>(h, dh, b, m, gA, gB, gBw, g, dh16, BH, S, Spad, D, dtype, st);
-        case MLSTM_DT_BF16:
-            return bwd_prep_dispatch<__nv_bfloat16>(h, dh, b, m, gA, gB, gBw, g, dh16, BH, S, Spad, D, dtype, st);
+        case MLSTM_DT_F32: PREP(float);
+        case MLSTM_DT_F16: PREP(__half);
+        case MLSTM_DT_BF16: PREP(__nv_bfloat16);
     }
+#undef PREP
     return MLSTM_E_ARG;
 }
 

@@ -181,7 +181,8 @@ int launch_state_scan(const void* U, const float* zU, const double* An_bound, co
                       cudaStream_t st, const double* late_bound = nullptr, float* rec = nullptr, size_t rec_stride = 0,
                       const double* summary = nullptr, void* statesT16 = nullptr, int reverse = 0, int* zero_word = nullptr);
 int launch_bwd_prep(const void* h, const void* dh, const float* b, const float* m, const float* gAn, float* gB,
-                    float* gBw, float* g, void* dh16, int BH, int S, int Spad, int D, int h_dtype, int dtype, cudaStream_t st);
+                    float* gBw, float* g, void* dh_out, const void* o, void* d_o, int BH, int S, int Spad, int D, int h_dtype,
+                    int dtype, cudaStream_t st);
 // dI, R: `nparts` partial vectors each, `part_stride` floats apart (see PassParams::dot_out).  scratch (optional,
 // gates_scratch_bytes(BH, Spad) bytes): long slices are then scanned in segments, one block each.
 int launch_df(const void* f, const float* dI, const float* R, void* df, void* di, int BH, int S, int Spad, int dtype,

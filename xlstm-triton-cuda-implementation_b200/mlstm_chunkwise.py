@@ -150,25 +150,45 @@ class ChunkSegment:
 
 def mlstm_chunkwise_backward(dh, q, k, v, f, i, h, m, b, chunk_size=256):
     """Gradients (dq, dk, dv, df, di) of the chunkwise forward without inbound state, in time linear in S."""
+    return _backward(dh, q, k, v, f, i, h, m, b, chunk_size)[:5]
+
+
+def _backward(dh, q, k, v, f, i, h, m, b, chunk_size, o=None):
+    """(dq, dk, dv, df, di, do).  With the output gate ``o``, dh is the gradient of h * silu(o)."""
+    if o is not None and (o.data_ptr() & 15):    # the fused gate derivative reads 16 bytes at a time
+        from .mlstm_matmul import output_gate_backward
+        dh, do = output_gate_backward(dh, h, o)
+        return _backward(dh, q, k, v, f, i, h, m, b, chunk_size)[:5] + (do,)
     dev = _lib.require_cuda(dh, q, k, v, f, i, h, m, b)
     B, NH, S, D = q.shape
     if dh.shape != q.shape or dh.dtype != h.dtype:
         raise ValueError("dh must match h in shape and element type")
     dt, hdt, chunk = _lib.dtype_code(q), _lib.dtype_code(h), int(chunk_size)
     L = _lib.lib()
-    nbytes = L.mlstm_chunk_bwd_workspace(B, NH, S, D, dt, hdt, chunk)
+    nbytes = (L.mlstm_chunk_bwd_workspace if o is None else L.mlstm_chunk_bwd_ogate_workspace)(B, NH, S, D, dt, hdt, chunk)
     if nbytes == 0:
         raise _lib.MlstmError(-4, "mlstm_chunk_bwd_workspace (needs float16/bfloat16, D = 128 or 256, chunk % 128 == 0)")
     ws = _lib.workspace(nbytes, dev)
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
     df, di = torch.empty_like(f), torch.empty_like(i)
+    do = None
+    if o is not None:
+        _lib.require_cuda(q, o)
+        do = torch.empty_like(o)
     with torch.cuda.device(dev):
-        rc = L.mlstm_chunk_bwd(dh.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), f.data_ptr(), i.data_ptr(), h.data_ptr(),
-                               m.data_ptr(), b.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), df.data_ptr(),
-                               di.data_ptr(), ws.data_ptr(), ws.numel(), B, NH, S, D, dt, hdt, chunk, _lib.stream_ptr(dev))
+        if o is not None:
+            rc = L.mlstm_chunk_bwd_ogate(dh.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), f.data_ptr(), i.data_ptr(),
+                                         h.data_ptr(), m.data_ptr(), b.data_ptr(), o.data_ptr(), dq.data_ptr(), dk.data_ptr(),
+                                         dv.data_ptr(), df.data_ptr(), di.data_ptr(), do.data_ptr(), ws.data_ptr(), ws.numel(),
+                                         B, NH, S, D, dt, hdt, chunk, _lib.stream_ptr(dev))
+        else:
+            rc = L.mlstm_chunk_bwd(dh.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), f.data_ptr(), i.data_ptr(),
+                                   h.data_ptr(), m.data_ptr(), b.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                                   df.data_ptr(), di.data_ptr(), ws.data_ptr(), ws.numel(), B, NH, S, D, dt, hdt, chunk,
+                                   _lib.stream_ptr(dev))
     _lib.check(rc, "mlstm_chunk_bwd")
     _lib.maybe_read_status(ws, dev, "mlstm_chunk_bwd")
-    return dq, dk, dv, df, di
+    return dq, dk, dv, df, di, do
 
 
 class _ChunkwiseWithGrad(torch.autograd.Function):

@@ -84,6 +84,14 @@ def mlstm_matmul_forward(q, k, v, f, i, h_dtype=torch.float32, flags=0):
 
 def mlstm_matmul_backward(dh, q, k, v, f, i, h, m, b, flags=0):
     """Run the backward; returns (dq, dk, dv, df, di) in the inputs' element type."""
+    return _backward(dh, q, k, v, f, i, h, m, b, flags)[:5]
+
+
+def _backward(dh, q, k, v, f, i, h, m, b, flags, o=None):
+    """(dq, dk, dv, df, di, do).  With the output gate ``o``, dh is the gradient of h * silu(o)."""
+    if o is not None and (o.data_ptr() & 15):    # the fused gate derivative reads 16 bytes at a time
+        dh, do = output_gate_backward(dh, h, o)
+        return _backward(dh, q, k, v, f, i, h, m, b, flags)[:5] + (do,)
     dev = _lib.require_cuda(dh, q, k, v, f, i, h, m, b)
     B, NH, S, D = q.shape
     if dh.shape != q.shape or dh.dtype != h.dtype:
@@ -92,15 +100,27 @@ def mlstm_matmul_backward(dh, q, k, v, f, i, h, m, b, flags=0):
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
     df, di = torch.empty_like(f), torch.empty_like(i)
     L = _lib.lib()
-    ws = _lib.workspace(L.mlstm_mm_bwd_workspace(B, NH, S, D, dt, hdt, flags), dev)
+    if o is None:
+        do = None
+        ws = _lib.workspace(L.mlstm_mm_bwd_workspace(B, NH, S, D, dt, hdt, flags), dev)
+    else:
+        _lib.require_cuda(q, o)
+        do = torch.empty_like(o)
+        ws = _lib.workspace(L.mlstm_mm_bwd_ogate_workspace(B, NH, S, D, dt, hdt, flags), dev)
     with torch.cuda.device(dev):
-        rc = L.mlstm_mm_bwd(dh.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), f.data_ptr(), i.data_ptr(),
-                            h.data_ptr(), m.data_ptr(), b.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-                            df.data_ptr(), di.data_ptr(), ws.data_ptr(), ws.numel(), B, NH, S, D, dt, hdt, flags,
-                            _lib.stream_ptr(dev))
+        if o is not None:
+            rc = L.mlstm_mm_bwd_ogate(dh.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), f.data_ptr(), i.data_ptr(),
+                                      h.data_ptr(), m.data_ptr(), b.data_ptr(), o.data_ptr(), dq.data_ptr(), dk.data_ptr(),
+                                      dv.data_ptr(), df.data_ptr(), di.data_ptr(), do.data_ptr(), ws.data_ptr(), ws.numel(), B,
+                                      NH, S, D, dt, hdt, flags, _lib.stream_ptr(dev))
+        else:
+            rc = L.mlstm_mm_bwd(dh.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), f.data_ptr(), i.data_ptr(),
+                                h.data_ptr(), m.data_ptr(), b.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                                df.data_ptr(), di.data_ptr(), ws.data_ptr(), ws.numel(), B, NH, S, D, dt, hdt, flags,
+                                _lib.stream_ptr(dev))
     _lib.check(rc, "mlstm_mm_bwd")
     _lib.maybe_read_status(ws, dev, "mlstm_mm_bwd")
-    return dq, dk, dv, df, di
+    return dq, dk, dv, df, di, do
 
 
 def output_gate_forward(h_inner, o):
@@ -152,11 +172,10 @@ class Triton_mLSTM(torch.autograd.Function):
         assert dh.is_contiguous()  # mlstm_matmul.py:385
         if ctx.gated:
             q, k, v, f, i, m, b, h, o = ctx.saved_tensors
-            dh, do = output_gate_backward(dh, h, o)
         else:
             q, k, v, f, i, m, b, h = ctx.saved_tensors
-            do = None
-        dq, dk, dv, df, di = mlstm_matmul_backward(dh, q, k, v, f, i, h, m, b, flags=_DEFAULT_FLAGS)
+            o = None
+        dq, dk, dv, df, di, do = _backward(dh, q, k, v, f, i, h, m, b, _DEFAULT_FLAGS, o)
         return dq, dk, dv, df, di, None, None, do
 
 

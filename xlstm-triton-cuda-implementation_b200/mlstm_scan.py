@@ -33,7 +33,8 @@ through the parallel kernels (``mlstm_matmul_backward``), whose cost is quadrati
 import torch
 
 from . import _lib
-from .mlstm_matmul import mlstm_matmul_backward, mlstm_matmul_forward, output_gate_backward, output_gate_forward
+from .mlstm_matmul import _backward as _matmul_backward
+from .mlstm_matmul import mlstm_matmul_forward, output_gate_backward, output_gate_forward
 
 __all__ = ["mlstm_scan", "output_gate_forward", "output_gate_backward"]
 
@@ -66,12 +67,11 @@ class _ScanWithGrad(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dh):
         q, k, v, f, i, o, m, b, h_inner = ctx.saved_tensors
-        dh_inner, do = output_gate_backward(dh.contiguous(), h_inner, o)
         if ctx.chunked:
-            from .mlstm_chunkwise import mlstm_chunkwise_backward
-            dq, dk, dv, df, di = mlstm_chunkwise_backward(dh_inner, q, k, v, f, i, h_inner, m, b, 256)
+            from .mlstm_chunkwise import _backward as backward
         else:
-            dq, dk, dv, df, di = mlstm_matmul_backward(dh_inner, q, k, v, f, i, h_inner, m, b, flags=ctx.flags)
+            backward = _matmul_backward
+        dq, dk, dv, df, di, do = backward(dh.contiguous(), q, k, v, f, i, h_inner, m, b, 256 if ctx.chunked else ctx.flags, o)
         return dq, dk, dv, df, di, do, None
 
 
