@@ -322,6 +322,7 @@ int launch_fwdc(const void* q, const void* k, const void* v, const void* o, void
     p.chunk_tiles = chunk / TILE; p.NB = w.NB; p.An_bound = w.An_bound; p.ident = w.ident;
     p.states = w.states; p.zstate = w.zstate;
     p.late_bound = late_bound;
+    if (chunk_pair_supported(D, dtype, p.chunk_tiles)) return launch_chunk_pair(FWDC, p, dtype, h_dtype, st);
     return launch_pass_tc(FWDC, p, dtype, h_dtype, st);
 }
 
@@ -533,9 +534,11 @@ static int chunk_bwd_impl(const void* dh, const void* q, const void* k, const vo
     p.col_rel = c.ga; p.col_w = c.gaw; p.col_ref = c.a_ref; p.row_rel = c.gAn; p.row_ref = c.An_ref;
     p.out = c.U; p.b_out = c.zU;
     if ((rc = launch_pass_tc(STATE, p, dtype, dtype, st)) != MLSTM_OK) return rc;
-    // inbound states of the blocks, transposed (dQ's state step contracts over the value dimension), and z
-    if ((rc = launch_state_scan(c.U, c.zU, c.An_bound, nullptr, nullptr, nullptr, c.zstate, nullptr, nullptr, BH, c.NB, D,
-                                dtype, st, nullptr, nullptr, 0, nullptr, w.statesT, 0)) != MLSTM_OK)
+    // Inbound states of the blocks and z.  dQ's state step contracts over the value dimension: the pair kernel reads the
+    // states as they are, the one-CTA kernel wants them transposed.
+    const bool pair = chunk_pair_supported(D, dtype, p.chunk_tiles);
+    if ((rc = launch_state_scan(c.U, c.zU, c.An_bound, nullptr, nullptr, pair ? w.statesT : nullptr, c.zstate, nullptr, nullptr, BH,
+                                c.NB, D, dtype, st, nullptr, nullptr, 0, nullptr, pair ? nullptr : w.statesT, 0)) != MLSTM_OK)
         return rc;
     // delta = dh . h, n, db -> the backward's per-row vectors (and dh in the input type)
     if ((rc = launch_bwd_prep(h, dh, b, m, c.gAn, w.gB, w.gBw, w.g, w.dh16, o, d_o, BH, S, Spad, D, h_dtype, dtype, st)) != MLSTM_OK)
@@ -559,27 +562,31 @@ static int chunk_bwd_impl(const void* dh, const void* q, const void* k, const vo
                        c.zU, S, Spad, c.NB, chunk, D);
         if (cudaGetLastError() != cudaSuccess) return MLSTM_E_CUDA;
     }
-    // the block recurrence in reverse: R_k [key, value] (for dV), its transpose (for dK) and r_k
+    // the block recurrence in reverse: R_k [key, value] (for dV and, in the pair kernel, for dK), its transpose (for dK in
+    // the one-CTA kernel) and r_k
     if ((rc = launch_state_scan(c.U, c.zU, c.An_bound, nullptr, nullptr, c.states, w.rvec, nullptr, nullptr, BH, c.NB, D,
-                                dtype, st, nullptr, nullptr, 0, nullptr, w.statesT2, 1)) != MLSTM_OK)
+                                dtype, st, nullptr, nullptr, 0, nullptr, pair ? nullptr : w.statesT2, 1)) != MLSTM_OK)
         return rc;
     // dQ = ((dH V^T + g_r) * decay) K within the block, + beta (S_k dh + g z_k) from the inbound state
+    auto pass = [&](int mode) {
+        return pair ? launch_chunk_pair(mode, p, dtype, dtype, st) : launch_pass_tc(mode, p, dtype, dtype, st);
+    };
     p.X = dhp; p.Y = v; p.Z = k;
     p.row_rel = w.gB; p.row_ref = c.An_ref; p.row_g = w.g; p.col_rel = c.ga; p.col_w = c.gaw; p.col_ref = c.a_ref; p.col_g = nullptr;
     p.states = w.statesT; p.zstate = c.zstate;
     p.out = dq; p.dot_src = q; p.dot_out = w.Rdot;
-    if ((rc = launch_pass_tc(DQC, p, dtype, dtype, st)) != MLSTM_OK) return rc;
+    if ((rc = pass(DQC)) != MLSTM_OK) return rc;
     // dK = ((V dH^T + g_c) * decay) Q within the block, + gamma (R_k v + r_k) from the later blocks
     p.X = v; p.Y = dhp; p.Z = q;
     p.row_rel = c.ga; p.row_ref = c.a_ref; p.row_g = nullptr; p.col_rel = w.gB; p.col_w = w.gBw; p.col_ref = c.An_ref; p.col_g = w.g;
-    p.states = w.statesT2; p.rvec = w.rvec;
+    p.states = pair ? c.states : w.statesT2; p.rvec = w.rvec;
     p.out = dk; p.dot_src = k; p.dot_out = w.dI;
-    if ((rc = launch_pass_tc(DKC, p, dtype, dtype, st)) != MLSTM_OK) return rc;
+    if ((rc = pass(DKC)) != MLSTM_OK) return rc;
     // dV = ((K Q^T) * decay / n) dH within the block, + gamma R_k^T k from the later blocks
     p.X = k; p.Y = q; p.Z = dhp;
     p.col_g = nullptr; p.states = c.states;
     p.out = dv; p.dot_src = nullptr; p.dot_out = nullptr;
-    if ((rc = launch_pass_tc(DVC, p, dtype, dtype, st)) != MLSTM_OK) return rc;
+    if ((rc = pass(DVC)) != MLSTM_OK) return rc;
     return launch_df(f, w.dI, w.Rdot, df, di, BH, S, Spad, dtype, st, TC_DOT_PARTS, static_cast<long long>(BH) * Spad, c.gscratch);
 }
 

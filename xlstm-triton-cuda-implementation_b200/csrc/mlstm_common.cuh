@@ -64,6 +64,7 @@ struct PassParams {
     const float* col_g;     // g per column (DK) or nullptr
     float er_add;           // constant term of er (FWD: log2(scale))
     void* out;           // [BH, S, D], element type chosen by the kernel template
+    void* out2;          // FWDC on CTA pairs: the result before the output gate (same type as out), or nullptr
     // FWD only
     const float* m;      // [BH, S] stabiliser, written by the gate pass
     float* b_out;        // [BH, S] row sums of the gated tile (the reference's B output) or nullptr
@@ -191,6 +192,9 @@ constexpr int TC_DOT_PARTS = 4;   // gate groups of the tensor-core passes
 int launch_pass_simt(int mode, const PassParams& p, int in_dtype, int out_dtype, cudaStream_t st);
 int launch_pass_tc(int mode, const PassParams& p, int in_dtype, int out_dtype, cudaStream_t st);
 bool tc_supported(int S, int D, int in_dtype);
+// chunkwise output and backward passes on CTA pairs (chunk_pair.cu); states: one row-major copy [key, value] for all modes
+bool chunk_pair_supported(int D, int in_dtype, int chunk_tiles);
+int launch_chunk_pair(int mode, const PassParams& p, int in_dtype, int out_dtype, cudaStream_t st);
 int launch_round_tf32(const void* in, void* out, long long n, cudaStream_t st);
 // fp32 [rows, D] -> bf16 [rows, 2 D] (hi | mid): the operands of the split tensor-core form (mm_tc.cu)
 int launch_split_bf16(const void* in, void* out, long long rows, int D, cudaStream_t st);

@@ -103,6 +103,21 @@ __device__ __forceinline__ void st_global_v8(void* p, uint32_t a0, uint32_t a1, 
                  : "memory");
 }
 
+// 16-byte read-only load that stays where it is written (the compiler may move an ordinary one down to its first use, behind
+// the waits it was meant to overlap)
+__device__ __forceinline__ uint4 ld_global_nc_v4(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+// Register share of the calling warpgroup (all four warps execute it).  An increase waits until the block's launch share
+// has that many to give: the shares must add up to no more than the launch's total.
+template <int N>
+__device__ __forceinline__ void set_max_regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void set_max_regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // brings the 128-byte line at p into L2 without occupying a register or a scoreboard slot
 __device__ __forceinline__ void prefetch_l2(const void* p) {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory");
