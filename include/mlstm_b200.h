@@ -191,6 +191,16 @@ int mlstm_chunk_apply(const void* q, const void* k, const void* v, const void* o
                       void* h, int h_dtype, float* S_out, float* z_out, void* workspace, size_t workspace_bytes, int B,
                       int NH, int S, int D, int dtype, int chunk, void* stream);
 
+/* The decoding step: S <= mlstm_step_max_tokens() positions of every sequence against a carried state, one launch, no
+ * workspace (the carry of mlstm_scan.py:143-195 position by position).  16-bit inputs, D = 128 or 256; everything inside
+ * is fp32, the gates double.  S_in, z_in [B*NH][D][D], [B*NH][D] fp32 stabilised by A_in; F_in, A_in [B*NH] double as in
+ * `carry_in` above (all four, or none: nothing carried in).  h of `h_dtype` (fp32 or the input type), times silu(o) when o
+ * is given.  The outputs S_out, z_out, F_out, A_out may each be NULL; they must not overlap the inputs. */
+int mlstm_step_max_tokens(void);
+int mlstm_step(const void* q, const void* k, const void* v, const void* f, const void* i, const void* o, const float* S_in,
+               const float* z_in, const double* F_in, const double* A_in, void* h, int h_dtype, float* S_out, float* z_out,
+               double* F_out, double* A_out, int B, int NH, int S, int D, int dtype, void* stream);
+
 /* Backward of the chunkwise forward, in time linear in S (the reference's scan is forward only, README.md:97;
  * the gradient formulas are those of mlstm_matmul.py:336-365 split into the part inside a block and the part
  * carried across blocks).  For a segment processed with no inbound state.

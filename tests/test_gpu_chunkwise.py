@@ -373,3 +373,31 @@ def test_sequence_parallel_over_nccl(gc):
     out = mp.Manager().dict()
     mp.spawn(_sp_worker, args=(world, port, x, out), nprocs=world, join=True)
     assert len(out) == world and all(e < TOL_16 for e in out.values()), dict(out)
+
+
+@pytest.mark.parametrize("D,dtype,T,gated", [
+    (128, torch.bfloat16, 1, True), (256, torch.float16, 1, False), (128, torch.float16, 4, True), (256, torch.bfloat16, 5, True),
+    (256, torch.bfloat16, 16, False), (128, torch.bfloat16, 17, True),      # 17: the first length that takes the blocks
+])
+def test_decoding_step_continues_a_segment(gc, D, dtype, T, gated):
+    """A prefix, then T positions in one call with the state carried in and out (csrc/step.cu up to 16 positions), then one
+    more, against the unsplit oracle.  16-bit inputs are exact in both; the prefix' state comes from the blocks."""
+    x = gc.make_inputs(2, 3, 300 + T + 1, D, dtype, f_mean=2.0, qkv_scale=D ** -0.5, seed=T + D)
+    o = torch.randn(x["q"].shape, generator=torch.Generator().manual_seed(T)).to(dtype)
+    ref = orc.matmul_forward(x["q"], x["k"], x["v"], x["f"], x["i"])
+    if gated:
+        ref = ref * torch.nn.functional.silu(o.double())
+    part = lambda a, b: [t[:, :, a:b].contiguous() for t in _dev(x)]
+    gate = lambda a, b: dict(o=o[:, :, a:b].contiguous().cuda()) if gated else {}
+    _, st = gc.PKG.mlstm_chunkwise(*part(0, 300), return_state=True)
+    h1, st1 = gc.PKG.mlstm_chunkwise(*part(300, 300 + T), initial=st, return_state=True, **gate(300, 300 + T))
+    h2, st2 = gc.PKG.mlstm_chunkwise(*part(300 + T, 301 + T), initial=st1, return_state=True, **gate(300 + T, 301 + T))
+    assert orc.max_abs_rel(torch.cat([h1, h2], 2), ref[:, :, 300:]) < TOL_16
+    _, whole = gc.PKG.mlstm_chunkwise(*_dev(x), return_state=True)
+    for a, b in zip(st2, whole):
+        assert a.shape == b.shape and a.dtype == b.dtype
+        assert orc.max_abs_rel(a, b.cpu()) < TOL_16
+    # T positions with nothing carried in: exact inputs, fp32 throughout (sums of at most D = 256 terms: 256 * 2^-24)
+    if T <= 16:
+        h0 = gc.PKG.mlstm_chunkwise(*part(0, T))
+        assert orc.max_abs_rel(h0, orc.matmul_forward(*(x[n][:, :, :T] for n in ("q", "k", "v", "f", "i")))) < 1e-4

@@ -88,6 +88,10 @@ def lib():
     L.mlstm_chunk_sp_local.argtypes = [vp] * 5 + [vp, sz] + [i32] * 6 + [vp]
     L.mlstm_chunk_sp_apply.restype = i32
     L.mlstm_chunk_sp_apply.argtypes = [vp] * 5 + [i32, i32, vp, i32, vp, vp, sz] + [i32] * 6 + [vp]
+    L.mlstm_step_max_tokens.restype = i32
+    L.mlstm_step_max_tokens.argtypes = []
+    L.mlstm_step.restype = i32
+    L.mlstm_step.argtypes = [vp] * 11 + [i32] + [vp] * 4 + [i32] * 5 + [vp]
     L.mlstm_chunk_read_mb.restype = i32
     L.mlstm_chunk_read_mb.argtypes = [vp, sz, vp, vp] + [i32] * 6 + [vp]
     L.mlstm_chunk_bwd_workspace.restype = sz
@@ -121,7 +125,7 @@ EXPORTS = [
     "mlstm_chunk_workspace", "mlstm_chunk_gate_summary", "mlstm_chunk_prepare", "mlstm_chunk_local_state",
     "mlstm_chunk_apply", "mlstm_chunk_sp_record_floats", "mlstm_chunk_sp_local", "mlstm_chunk_sp_apply",
     "mlstm_chunk_read_mb", "mlstm_chunk_bwd_workspace", "mlstm_chunk_bwd",
-    "mlstm_forward_f16_static_status", "mlstm_selftest_wait_timeout", "mlstm_ogate_fwd", "mlstm_ogate_bwd",
+    "mlstm_step_max_tokens", "mlstm_step", "mlstm_forward_f16_static_status", "mlstm_selftest_wait_timeout", "mlstm_ogate_fwd", "mlstm_ogate_bwd",
 ]
 
 

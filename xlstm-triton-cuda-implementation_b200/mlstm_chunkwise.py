@@ -111,6 +111,30 @@ class ChunkSegment:
         _lib.maybe_read_status(self.ws, self.dev, "mlstm_chunk_apply")
         return (h, (S_out, z_out)) if return_state else h
 
+    def step(self, initial=None, h_dtype=torch.float32, return_state=False):
+        """The whole segment in one launch, for the few positions of a decoding step (S <= mlstm_step_max_tokens):
+        h, or (h, (S, z, F, A)) with ``return_state``.  ``initial`` as in ``mlstm_chunkwise``."""
+        BH = self.B * self.NH
+        h = torch.empty((self.B, self.NH, self.S, self.D), dtype=h_dtype, device=self.dev)
+        carried = [None] * 4
+        if initial is not None:
+            carried = [x.to(device=self.dev, dtype=d).contiguous()
+                       for x, d in zip(initial, (torch.float32, torch.float32, torch.float64, torch.float64))]
+            if [x.numel() for x in carried] != [BH * self.D * self.D, BH * self.D, BH, BH]:
+                raise ValueError("initial must be (S [B*NH, D, D], z [B*NH, D], F [B*NH], A [B*NH])")
+        out = [None] * 4
+        if return_state:
+            gates = torch.empty((2, BH), dtype=torch.float64, device=self.dev)
+            out = [torch.empty((BH, self.D, self.D), dtype=torch.float32, device=self.dev),
+                   torch.empty((BH, self.D), dtype=torch.float32, device=self.dev), gates[0], gates[1]]
+        ptr = lambda t: t.data_ptr() if t is not None else None
+        with torch.cuda.device(self.dev):
+            rc = self.L.mlstm_step(self.q.data_ptr(), self.k.data_ptr(), self.v.data_ptr(), self.f.data_ptr(),
+                                   self.i.data_ptr(), ptr(self.o), *map(ptr, carried), h.data_ptr(), _lib.dtype_code(h),
+                                   *map(ptr, out), self.B, self.NH, self.S, self.D, self.dt, self._stream())
+        _lib.check(rc, "mlstm_step")
+        return (h, tuple(out)) if return_state else h
+
     def read_mb(self):
         """After ``apply``: the stabiliser m and the row sums b [B, NH, S] float32 (the parallel forward's M, B)."""
         m = torch.empty((self.B, self.NH, self.S), dtype=torch.float32, device=self.dev)
@@ -225,6 +249,9 @@ def mlstm_chunkwise(q, k, v, f, i, chunk_size=256, h_dtype=torch.float32, initia
             raise ValueError("gradients are available for the plain call: no initial / return_state / o, float32 h")
         return _ChunkwiseWithGrad.apply(q, k, v, f, i, int(chunk_size))
     seg = ChunkSegment(q, k, v, f, i, chunk_size, shared_workspace=True, o=o)
+    # a decoding step: one launch and fp32 throughout instead of the five launches of a block of 256 (csrc/step.cu)
+    if seg.S <= seg.L.mlstm_step_max_tokens():
+        return seg.step(initial, h_dtype=h_dtype, return_state=return_state)
     carry = None
     state_in = None
     if initial is not None:
