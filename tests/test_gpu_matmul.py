@@ -347,3 +347,44 @@ def test_argument_errors(gc):
     x = gc.make_inputs(1, 1, 64, 32, torch.float32)
     with pytest.raises(gc._lib.MlstmError):
         gc.run_forward(x, flags=gc._lib.F_FORCE_TC)  # fp32 at D = 32 has no tensor-core path
+
+
+@pytest.mark.parametrize("BH,S,D,gated,pad", [
+    (64, 2048, 128, False, 0),      # the smallest that takes the chunkwise form
+    (33, 4001, 256, True, 0),       # ragged last block, an odd number of tiles
+    (66, 2049, 128, False, 640),    # one position in the last block; input gates of -inf in front (left padding)
+])
+def test_long_sequences_take_the_chunkwise_form(gc, BH, S, D, gated, pad):
+    """The parallel entry points' chunkwise route against the oracle (first and last slice) and against the quadratic kernel,
+    whose error it may not exceed by more than the noise of the measure (a quarter)."""
+    dt = torch.bfloat16
+    x = gc.make_inputs(1, BH, S, D, dt, f_mean=3.0, qkv_scale=D ** -0.5, seed=S, with_o=gated)
+    if pad:
+        x["i"][:, :, :pad] = -float("inf")
+    dev = {n: t.cuda() for n, t in x.items()}
+    args = [dev[n] for n in ("q", "k", "v", "f", "i")]
+    res = []
+    for flags in (0, gc._lib.F_FORCE_TC):
+        h, m, b = gc.PKG.mlstm_matmul_forward(*args, flags=flags)
+        if pad:
+            h[:, :, :pad] = 0.0          # rows without a finite gate have no value
+            dev["dh"][:, :, :pad] = 0.0
+        gr = None if pad else gc.PKG.mlstm_matmul.__globals__["_backward"](dev["dh"], *args, h, m, b, flags, dev.get("o"))
+        res.append((h, m, b, gr))
+    (h, m, b, gr), (h2, m2, b2, gr2) = res
+    for sl in (0, BH - 1):
+        y = {n: t[:, sl:sl + 1, pad:] for n, t in x.items()}
+        ref, _, b_ref, _ = orc.matmul_forward(y["q"], y["k"], y["v"], y["f"], y["i"], return_state=True)
+        err = lambda t, r: float((t.double().cpu() - r).norm() / r.norm())
+        cut = lambda t: t[:, sl:sl + 1, pad:]
+        assert err(cut(h), ref) < 1.25 * err(cut(h2), ref)
+        if gr is None:
+            continue
+        sg = torch.sigmoid(y["o"].double()) if gated else None
+        dh = y["dh"].double() * (y["o"].double() * sg if gated else 1.0)
+        refs = list(orc.matmul_backward(dh, y["q"], y["k"], y["v"], y["f"], y["i"]))
+        refs[3][..., 0] = 0.0
+        if gated:
+            refs.append(y["dh"].double() * ref * sg * (1.0 + y["o"].double() * (1.0 - sg)))
+        for name, a, a2, r in zip(("dq", "dk", "dv", "df", "di", "do"), gr, gr2, refs):
+            assert err(cut(a), r) < 1.25 * err(cut(a2), r), name

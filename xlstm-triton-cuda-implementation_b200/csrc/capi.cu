@@ -281,6 +281,7 @@ size_t mlstm_mm_fwd_workspace(int B, int NH, int S, int D, int dtype, int flags)
     // (sized for float32 h; a 16-bit h at these head dimensions takes the smaller one-pass workspace)
     if (mm_fwd_two_pass(S, D, dtype, MLSTM_DT_F32, flags))
         return carve_fwd(nullptr, B * NH, S, false).bytes + two_pass_extra_bytes(B * NH, S, dtype);
+    if (mm_chunk_route(B * NH, S, D, dtype, flags)) return mm_chunk_fwd_bytes(B * NH, S, D);
     return carve_fwd(nullptr, B * NH, S, false).bytes + tf32_copy_bytes(B * NH, S, D, dtype, flags, 3);
 }
 
@@ -299,6 +300,10 @@ int mlstm_mm_fwd(const void* q, const void* k, const void* v, const void* f, con
         return two_pass_forward(q, k, v, f, i, nullptr, static_cast<float*>(h), m, b, w, static_cast<uint8_t*>(workspace) + w.bytes,
                                 B * NH, S, D, dtype, static_cast<cudaStream_t>(stream));
     }
+    if (mm_chunk_route(B * NH, S, D, dtype, flags)) {
+        if (!workspace || workspace_bytes < mm_chunk_fwd_bytes(B * NH, S, D) || !aligned16(workspace)) return MLSTM_E_WORKSPACE;
+        return mm_chunk_fwd(q, k, v, f, i, h, m, b, workspace, B * NH, S, D, dtype, h_dtype, static_cast<cudaStream_t>(stream));
+    }
     const size_t extra = tf32_copy_bytes(B * NH, S, D, dtype, flags, 3);
     if (!workspace || workspace_bytes < w.bytes + extra || !aligned16(workspace)) return MLSTM_E_WORKSPACE;
     return forward_impl(q, k, v, f, i, nullptr, h, m, b, w, B * NH, S, D, dtype, h_dtype, flags,
@@ -314,6 +319,7 @@ static int dh_copy_bytes(int dtype, int h_dtype, bool gated) {
 
 static size_t mm_bwd_workspace(int B, int NH, int S, int D, int dtype, int h_dtype, int flags, bool gated) {
     if (check_dims(B, NH, S, D) != MLSTM_OK) return 0;
+    if (mm_chunk_route(B * NH, S, D, dtype, flags)) return mm_chunk_bwd_bytes(B * NH, S, D, dh_copy_bytes(dtype, h_dtype, gated) != 0);
     const size_t own = carve_bwd(nullptr, B * NH, S, D, dh_copy_bytes(dtype, h_dtype, gated)).bytes;
     if (mm_bwd_two_pass(S, D, dtype, flags)) return own + two_pass_bwd_extra_bytes(B * NH, S, D, dtype);
     return own + tf32_copy_bytes(B * NH, S, D, dtype, flags, 4);
@@ -340,8 +346,12 @@ static int mm_bwd_impl(const void* dh, const void* q, const void* k, const void*
         return MLSTM_E_ALIGN;
     const int BH = B * NH, Spad = round_up(S, TILE);
     const int dh_es = dh_copy_bytes(dtype, h_dtype, o != nullptr);
-    BwdWs w = carve_bwd(workspace, BH, S, D, dh_es);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (mm_chunk_route(B * NH, S, D, dtype, flags)) {
+        if (!workspace || workspace_bytes < mm_chunk_bwd_bytes(BH, S, D, dh_es != 0) || !aligned16(workspace)) return MLSTM_E_WORKSPACE;
+        return mm_chunk_bwd(dh, q, k, v, f, i, h, m, b, o, d_o, dq, dk, dv, df, di, workspace, BH, S, D, dtype, h_dtype, st);
+    }
+    BwdWs w = carve_bwd(workspace, BH, S, D, dh_es);
     if (mm_bwd_two_pass(S, D, dtype, flags)) {
         if (!workspace || workspace_bytes < w.bytes + two_pass_bwd_extra_bytes(BH, S, D, dtype) || !aligned16(workspace))
             return MLSTM_E_WORKSPACE;

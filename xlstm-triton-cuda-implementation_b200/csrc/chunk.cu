@@ -9,7 +9,8 @@
 //     S_{k+1} = exp(A_end(k-1) - A_end(k)) S_k + U_k,    U_k = sum_{j in block k} exp(a_j - A_end(k)) k_j v_j^T
 // (S is indexed [key, value]; z is the same with v dropped: the normaliser vector).  A query t of block k
 // gets   num_t = intra-block part + exp(A_end(k-1) - A_t) (q_t S_k) / sqrt(D)   and the same for b_t.
-// Both contractions run on the tensor-core pass kernel (modes STATE and FWDC, mm_tc.cu).
+// The contributions U_k come from chunk_state.cu, the output from mode FWDC of chunk_pair.cu (mm_tc.cu for an odd number of
+// tiles per block).
 #include "mlstm_common.cuh"
 
 namespace mlstm {
@@ -78,7 +79,7 @@ state_scan_kernel(const T16* __restrict__ U, const float* __restrict__ zU, const
     const int off = is_vec ? ((blockIdx.x - npatch) * SCAN_THREADS_S + threadIdx.x) * 4 : (prow0 + lrow) * D + pcol0 + lcol;
     const bool valid = !is_vec || off < D;     // threads past the end still help with the factor tables and the barriers
     const size_t per_block = is_vec ? D : DD;
-    // block contributions: the matrices in the 16-bit input type (as the tensor-core pass wrote them), the vectors in fp32
+    // block contributions: the matrices as the tensor-core pass wrote them, the vectors in fp32
     const float* srcz = zU + static_cast<size_t>(bh) * NB * per_block + off;
     const T16* srcU = U + static_cast<size_t>(bh) * NB * per_block + off;
     const float* init = is_vec ? z_in : S_in;
@@ -171,43 +172,6 @@ state_scan_kernel(const T16* __restrict__ U, const float* __restrict__ zU, const
     if (dst) *reinterpret_cast<float4*>(dst + static_cast<size_t>(bh) * stride + off) = s;
 }
 
-// Vector part of what block k contributes to the backward's carried state:
-//   p_k[d] = sum_{t in block k} beta_t g_t q_t[d],  beta_t = exp(A_end(k-1) - A_t) scale / n_t,  g_t = db_t n_t
-// (the matrix part sum_t beta_t q_t dh_t^T comes from the tensor-core STATE pass).  One block of D threads per
-// (block, slice); log2 beta_t = gB_rel[t] + An_ref[t / 64] - bound[k] with the vectors of the backward preparation.
-// The weights beta_t g_t of the block's positions are computed once (into shared memory), then every thread adds up
-// its dimension over them: evaluated per thread and position they were most of the kernel.
-constexpr int RVEC_MAX_CHUNK = 2048;   // positions of a block whose weights fit the table; longer blocks take several rounds
-
-template <typename T16>
-__global__ void rvec_partial_kernel(const T16* __restrict__ q, const float* __restrict__ gB_rel,
-                                    const double* __restrict__ An_ref, const double* __restrict__ An_bound,
-                                    const float* __restrict__ g, float* __restrict__ out, int S, int Spad, int NB, int chunk,
-                                    int D) {
-    grid_dep_wait();
-    grid_dep_launch();
-    __shared__ float wt[RVEC_MAX_CHUNK];
-    const int k = blockIdx.x, bh = blockIdx.y, d = threadIdx.x;
-    const double b0 = An_bound[static_cast<size_t>(bh) * (NB + 1) + k];
-    const int t0 = k * chunk, t1 = min(t0 + chunk, S);
-    float acc = 0.0f;
-    for (int r0 = t0; r0 < t1; r0 += RVEC_MAX_CHUNK) {
-        const int rn = min(RVEC_MAX_CHUNK, t1 - r0);
-        __syncthreads();
-        for (int j = threadIdx.x; j < rn; j += blockDim.x) {
-            const int t = r0 + j;
-            const size_t vi = static_cast<size_t>(bh) * Spad + t;
-            const float e = gB_rel[vi] + static_cast<float>(An_ref[static_cast<size_t>(bh) * (Spad / REF_BLOCK) + t / REF_BLOCK] - b0);
-            wt[j] = exp2f(e) * g[vi];   // exp2(-inf) = 0 for the first block when nothing is carried in
-        }
-        __syncthreads();
-        const T16* qp = q + (static_cast<size_t>(bh) * S + r0) * D + d;
-#pragma unroll 8
-        for (int j = 0; j < rn; j++) acc = fmaf(wt[j], to_f32<T16>(qp[static_cast<size_t>(j) * D]), acc);
-    }
-    out[(static_cast<size_t>(bh) * NB + k) * D + d] = acc;
-}
-
 // Sequence-parallel fold: from the gathered records of all segments (per slice: S | z | {F_end, A_end},
 // every segment's state stabilised by its OWN prefix maximum and its F counted from zero) to the
 // inbound state of segment `rank` and its late carry.  With F_in(g) the log-forget total before
@@ -262,7 +226,9 @@ struct ChunkWs {
     size_t bytes;
 };
 
-ChunkWs carve(void* ws, int BH, int S, int D, int chunk) {
+// parts: 16-bit matrices a carried state is held in.  2: written by launch_carried_states, and what only the stages of
+// the 1-part form use is left out
+ChunkWs carve(void* ws, int BH, int S, int D, int chunk, int parts = 1) {
     ChunkWs w{};
     uint8_t* base = static_cast<uint8_t*>(ws);
     size_t off = 0;
@@ -286,16 +252,20 @@ ChunkWs carve(void* ws, int BH, int S, int D, int chunk) {
     w.An_bound = static_cast<double*>(take(static_cast<size_t>(BH) * (w.NB + 1) * sizeof(double)));
     const size_t gs = gates_scratch_bytes(BH, static_cast<int>(Spad));
     w.gscratch = gs ? static_cast<double*>(take(gs)) : nullptr;
-    w.ident = take(static_cast<size_t>(D) * D * 2);
-    w.U = take(nblk * D * D * 2);
-    w.zU = static_cast<float*>(take(nblk * D * sizeof(float)));
-    w.states = take(nblk * D * D * 2);
+    if (parts == 1) {
+        w.ident = take(static_cast<size_t>(D) * D * 2);
+        w.U = take(nblk * D * D * 2);
+        w.zU = static_cast<float*>(take(nblk * D * sizeof(float)));
+    }
+    w.states = take(nblk * D * D * 2 * parts);
     w.zstate = static_cast<float*>(take(nblk * D * sizeof(float)));
-    // sequence-parallel stages: this segment's gate summary, the folded inbound state and the late carry
-    w.summary = static_cast<double*>(take(static_cast<size_t>(BH) * 2 * sizeof(double)));
-    w.late = static_cast<double*>(take(static_cast<size_t>(BH) * sizeof(double)));
-    w.S_in = static_cast<float*>(take(static_cast<size_t>(BH) * D * D * sizeof(float)));
-    w.z_in = static_cast<float*>(take(static_cast<size_t>(BH) * D * sizeof(float)));
+    if (parts == 1) {
+        // sequence-parallel stages: this segment's gate summary, the folded inbound state and the late carry
+        w.summary = static_cast<double*>(take(static_cast<size_t>(BH) * 2 * sizeof(double)));
+        w.late = static_cast<double*>(take(static_cast<size_t>(BH) * sizeof(double)));
+        w.S_in = static_cast<float*>(take(static_cast<size_t>(BH) * D * D * sizeof(float)));
+        w.z_in = static_cast<float*>(take(static_cast<size_t>(BH) * D * sizeof(float)));
+    }
     w.bytes = off;
     return w;
 }
@@ -309,9 +279,18 @@ int check_chunk_args(int B, int NH, int S, int D, int dtype, int chunk) {
     return MLSTM_OK;
 }
 
+// arguments of the forward's states (chunk_state.cu): X = K, Y = V, and z, the same with V dropped
+BlockStateArgs forward_states(const void* k, const void* v, const ChunkWs& w, int BH, int S, int Spad, int chunk) {
+    BlockStateArgs a{};
+    a.X = k; a.Y = v; a.col_w = w.gaw; a.col_ref = w.a_ref; a.An_bound = w.An_bound;
+    a.S = S; a.Spad = Spad; a.BH = BH; a.NB = w.NB; a.chunk = chunk; a.status = w.status;
+    a.U = w.U; a.vec = w.zU;
+    return a;
+}
+
 // h of the segment from the per-block inbound states (FWDC pass)
 int launch_fwdc(const void* q, const void* k, const void* v, const void* o, void* h, int h_dtype, const ChunkWs& w, int BH,
-                int S, int Spad, int D, int dtype, int chunk, const double* late_bound, cudaStream_t st) {
+                int S, int Spad, int D, int dtype, int chunk, const double* late_bound, cudaStream_t st, int parts = 1) {
     PassParams p{};
     p.S = S; p.Spad = Spad; p.BH = BH; p.D = D; p.status = w.status; p.sched = w.status + 8;
     p.sched_zeroed = 1;   // by the state scan in front of this pass
@@ -322,6 +301,7 @@ int launch_fwdc(const void* q, const void* k, const void* v, const void* o, void
     p.chunk_tiles = chunk / TILE; p.NB = w.NB; p.An_bound = w.An_bound; p.ident = w.ident;
     p.states = w.states; p.zstate = w.zstate;
     p.late_bound = late_bound;
+    p.state_parts = parts;
     if (chunk_pair_supported(D, dtype, p.chunk_tiles)) return launch_chunk_pair(FWDC, p, dtype, h_dtype, st);
     return launch_pass_tc(FWDC, p, dtype, h_dtype, st);
 }
@@ -405,17 +385,8 @@ int mlstm_chunk_prepare(const void* k, const void* v, const void* f, const void*
     if ((rc = launch_gates_fwd(f, i, w.ga, w.gAn, w.a_ref, w.An_ref, w.m, BH, S, Spad, dtype, st, carry_in, summary_out,
                                w.An_bound, chunk, w.gscratch, w.gaw, w.status, STATUS_WORDS)) != MLSTM_OK)
         return rc;
-    if ((rc = launch_identity(w.ident, D, dtype, st)) != MLSTM_OK) return rc;
-    // U_k[key, value] = sum_j exp(a_j - A_end(k)) k_j[key] v_j[value];  zU_k[key] = sum_j exp(...) k_j[key]
-    PassParams p{};
-    p.S = S; p.Spad = Spad; p.BH = BH; p.D = D; p.status = w.status; p.sched = w.status + 8; p.sched_zeroed = 1;
-    p.X = k;  // unused by STATE (the stationary operand is the identity); keeps the tensor map valid
-    p.Y = k; p.Z = v;
-    p.col_rel = w.ga; p.col_w = w.gaw; p.col_ref = w.a_ref;
-    p.row_rel = w.gAn; p.row_ref = w.An_ref;  // unused by STATE
-    p.out = w.U; p.b_out = w.zU;
-    p.chunk_tiles = chunk / TILE; p.NB = w.NB; p.An_bound = w.An_bound; p.ident = w.ident;
-    return launch_pass_tc(STATE, p, dtype, dtype, st);
+    if (!chunk_pair_supported(D, dtype, chunk / TILE) && (rc = launch_identity(w.ident, D, dtype, st)) != MLSTM_OK) return rc;
+    return launch_block_states(forward_states(k, v, w, BH, S, Spad, chunk), D, dtype, st);
 }
 
 int mlstm_chunk_local_state(void* workspace, size_t workspace_bytes, float* S_end, float* z_end, int B, int NH, int S,
@@ -459,19 +430,21 @@ int mlstm_chunk_apply(const void* q, const void* k, const void* v, const void* o
 // the tensor-core pass); across blocks dQ uses the forward's inbound state S_k, and dK, dV use a state
 // carried BACK over the blocks,
 //   R_k = sum_{t after block k} exp(A_end(k) - A_t) (scale / n_t) q_t dh_t^T   (+ the vector r_k with g_t q_t),
-// built like the forward states: per-block contributions from one STATE pass (Y = Q, Z = dH, column
+// built like the forward states: per-block contributions from chunk_state.cu (X = Q, Y = dH, column
 // weights from the backward preparation), then the block recurrence walked in reverse.  dI and the row
 // sums behind dF are row dots of the complete fp32 accumulators, as in the parallel backward
 // (mlstm_matmul.py:256-316, 319-333 give the quantities; the reference has no chunkwise backward).
 struct ChunkBwdWs {
     ChunkWs f;
     float *gB, *gBw, *g, *dI, *Rdot, *rvec;
-    void *dh16, *statesT, *statesT2;
+    void *dh16;
+    void *fstates;     // the forward's inbound states (1 part: transposed, for the one-CTA kernel)
+    void *rstatesT;    // 1 part: transposed copy of the states carried back
     size_t bytes;
 };
-static ChunkBwdWs carve_bwd_chunk(void* ws, int BH, int S, int D, int chunk, bool need_dh16) {
+static ChunkBwdWs carve_bwd_chunk(void* ws, int BH, int S, int D, int chunk, bool need_dh16, int parts = 1) {
     ChunkBwdWs w{};
-    w.f = carve(ws, BH, S, D, chunk);
+    w.f = carve(ws, BH, S, D, chunk, parts);
     uint8_t* base = static_cast<uint8_t*>(ws);
     size_t off = w.f.bytes;
     auto take = [&](size_t bytes) {
@@ -487,8 +460,8 @@ static ChunkBwdWs carve_bwd_chunk(void* ws, int BH, int S, int D, int chunk, boo
     w.dI = static_cast<float*>(take(vec * TC_DOT_PARTS));     // partial row dots, one per gate group
     w.Rdot = static_cast<float*>(take(vec * TC_DOT_PARTS));
     w.rvec = static_cast<float*>(take(nblk * D * sizeof(float)));
-    w.statesT = take(nblk * D * D * 2);
-    w.statesT2 = take(nblk * D * D * 2);
+    w.fstates = take(nblk * D * D * 2 * parts);
+    w.rstatesT = parts == 1 ? take(nblk * D * D * 2) : nullptr;
     w.dh16 = need_dh16 ? take(static_cast<size_t>(BH) * S * D * 2) : nullptr;
     w.bytes = off;
     return w;
@@ -504,6 +477,77 @@ size_t mlstm_chunk_bwd_ogate_workspace(int B, int NH, int S, int D, int dtype, i
     return carve_bwd_chunk(nullptr, B * NH, S, D, chunk, true).bytes;
 }
 
+// (arguments checked, workspace carved by the caller)
+static int chunk_bwd_core(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h,
+                          const float* m, const float* b, const void* o, void* d_o, void* dq, void* dk, void* dv, void* df, void* di,
+                          const ChunkBwdWs& w, int BH, int S, int D, int dtype, int h_dtype, int chunk, int parts, cudaStream_t st) {
+    const int Spad = round_up(S, TILE);
+    const ChunkWs& c = w.f;
+    int rc;
+    // gates and forward states, as in the forward (the gate pass also clears the status word and the work-item counters)
+    if ((rc = launch_gates_fwd(f, i, c.ga, c.gAn, c.a_ref, c.An_ref, nullptr, BH, S, Spad, dtype, st, nullptr, nullptr,
+                               c.An_bound, chunk, c.gscratch, c.gaw, c.status, STATUS_WORDS)) != MLSTM_OK)
+        return rc;
+    // Two parts: every pass on CTA pairs, which read the states as they are.  One part: dQ and dK on the one-CTA kernel (its
+    // state step contracts over transposed states).  df is a running sum of differences of the row dots of these two passes,
+    // in which the rounding of a 16-bit state's path adds up (1 to 4 % of df at S = 16384, whatever the order): this entry
+    // keeps the rounding it has always had there, and with it its results.
+    const bool two = parts == 2;
+    BlockStateArgs fwd = forward_states(k, v, c, BH, S, Spad, chunk);
+    if (two) {
+        fwd.U = w.fstates; fwd.vec = c.zstate;
+        if ((rc = launch_carried_states(fwd, D, dtype, st)) != MLSTM_OK) return rc;
+    } else {
+        if ((rc = launch_identity(c.ident, D, dtype, st)) != MLSTM_OK) return rc;
+        if ((rc = launch_block_states(fwd, D, dtype, st)) != MLSTM_OK) return rc;
+        if ((rc = launch_state_scan(c.U, c.zU, c.An_bound, nullptr, nullptr, nullptr, c.zstate, nullptr, nullptr, BH, c.NB, D, dtype, st,
+                                    nullptr, nullptr, 0, nullptr, w.fstates, 0)) != MLSTM_OK)
+            return rc;
+    }
+    // delta = dh . h, n, db -> the backward's per-row vectors (and dh in the input type)
+    if ((rc = launch_bwd_prep(h, dh, b, m, c.gAn, w.gB, w.gBw, w.g, w.dh16, o, d_o, BH, S, Spad, D, h_dtype, dtype, st)) != MLSTM_OK)
+        return rc;
+    const void* dhp = w.dh16 ? w.dh16 : dh;
+    // the state carried back, R_k [key, value] and r_k: the recurrence in reverse over what every block contributes,
+    // P_k = sum_t beta_t q_t dh_t^T, p_k = sum_t beta_t g_t q_t with beta_t = exp(A_end(k-1) - A_t) scale / n_t, g_t = db_t n_t
+    BlockStateArgs bwd = fwd;
+    bwd.X = q; bwd.Y = dhp; bwd.col_w = w.gBw; bwd.col_ref = c.An_ref; bwd.col_g = w.g; bwd.reverse = 1;
+    if (two) {
+        bwd.U = c.states; bwd.vec = w.rvec;
+        if ((rc = launch_carried_states(bwd, D, dtype, st)) != MLSTM_OK) return rc;
+    } else {
+        if ((rc = launch_block_states(bwd, D, dtype, st)) != MLSTM_OK) return rc;
+        if ((rc = launch_state_scan(c.U, c.zU, c.An_bound, nullptr, nullptr, c.states, w.rvec, nullptr, nullptr, BH, c.NB, D, dtype, st,
+                                    nullptr, nullptr, 0, nullptr, w.rstatesT, 1)) != MLSTM_OK)
+            return rc;
+    }
+    PassParams p{};
+    p.S = S; p.Spad = Spad; p.BH = BH; p.D = D; p.status = c.status; p.sched = c.status + 8; p.sched_zeroed = 1;
+    p.chunk_tiles = chunk / TILE; p.NB = c.NB; p.An_bound = c.An_bound; p.ident = c.ident; p.state_parts = parts;
+    p.dot_part_stride = static_cast<long long>(BH) * Spad;
+    // dQ = ((dH V^T + g_r) * decay) K within the block, + beta (S_k dh + g z_k) from the inbound state
+    auto pass = [&](int mode, bool pair) {
+        return pair ? launch_chunk_pair(mode, p, dtype, dtype, st) : launch_pass_tc(mode, p, dtype, dtype, st);
+    };
+    p.X = dhp; p.Y = v; p.Z = k;
+    p.row_rel = w.gB; p.row_ref = c.An_ref; p.row_g = w.g; p.col_rel = c.ga; p.col_w = c.gaw; p.col_ref = c.a_ref; p.col_g = nullptr;
+    p.states = w.fstates; p.zstate = c.zstate;
+    p.out = dq; p.dot_src = q; p.dot_out = w.Rdot;
+    if ((rc = pass(DQC, two)) != MLSTM_OK) return rc;
+    // dK = ((V dH^T + g_c) * decay) Q within the block, + gamma (R_k v + r_k) from the later blocks
+    p.X = v; p.Y = dhp; p.Z = q;
+    p.row_rel = c.ga; p.row_ref = c.a_ref; p.row_g = nullptr; p.col_rel = w.gB; p.col_w = w.gBw; p.col_ref = c.An_ref; p.col_g = w.g;
+    p.states = two ? c.states : w.rstatesT; p.rvec = w.rvec;
+    p.out = dk; p.dot_src = k; p.dot_out = w.dI;
+    if ((rc = pass(DKC, two)) != MLSTM_OK) return rc;
+    // dV = ((K Q^T) * decay / n) dH within the block, + gamma R_k^T k from the later blocks
+    p.X = k; p.Y = q; p.Z = dhp;
+    p.col_g = nullptr; p.states = c.states;
+    p.out = dv; p.dot_src = nullptr; p.dot_out = nullptr;
+    if ((rc = pass(DVC, chunk_pair_supported(D, dtype, p.chunk_tiles))) != MLSTM_OK) return rc;
+    return launch_df(f, w.dI, w.Rdot, df, di, BH, S, Spad, dtype, st, TC_DOT_PARTS, static_cast<long long>(BH) * Spad, c.gscratch);
+}
+
 static int chunk_bwd_impl(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h,
                           const float* m, const float* b, const void* o, void* d_o, void* dq, void* dk, void* dv, void* df, void* di,
                           void* workspace, size_t workspace_bytes, int B, int NH, int S, int D, int dtype, int h_dtype, int chunk,
@@ -515,79 +559,11 @@ static int chunk_bwd_impl(const void* dh, const void* q, const void* k, const vo
     if (!aligned16(dh) || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(h) || !aligned16(dq) ||
         !aligned16(dk) || !aligned16(dv))
         return MLSTM_E_ALIGN;
-    const int BH = B * NH, Spad = round_up(S, TILE);
-    const bool need16 = o || h_dtype != dtype;   // dh in the input type, taken through the output gate where there is one
-    ChunkBwdWs w = carve_bwd_chunk(workspace, BH, S, D, chunk, need16);
+    // dh in the input type, taken through the output gate where there is one
+    ChunkBwdWs w = carve_bwd_chunk(workspace, B * NH, S, D, chunk, o || h_dtype != dtype);
     if (!workspace || workspace_bytes < w.bytes || !aligned16(workspace)) return MLSTM_E_WORKSPACE;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const ChunkWs& c = w.f;
-    // gates and forward states, as in the forward (the gate pass also clears the status word and the work-item counters)
-    if ((rc = launch_gates_fwd(f, i, c.ga, c.gAn, c.a_ref, c.An_ref, nullptr, BH, S, Spad, dtype, st, nullptr, nullptr,
-                               c.An_bound, chunk, c.gscratch, c.gaw, c.status, STATUS_WORDS)) != MLSTM_OK)
-        return rc;
-    if ((rc = launch_identity(c.ident, D, dtype, st)) != MLSTM_OK) return rc;
-    PassParams p{};
-    p.S = S; p.Spad = Spad; p.BH = BH; p.D = D; p.status = c.status; p.sched = c.status + 8; p.sched_zeroed = 1;
-    p.chunk_tiles = chunk / TILE; p.NB = c.NB; p.An_bound = c.An_bound; p.ident = c.ident;
-    p.dot_part_stride = static_cast<long long>(BH) * Spad;
-    p.X = k; p.Y = k; p.Z = v;
-    p.col_rel = c.ga; p.col_w = c.gaw; p.col_ref = c.a_ref; p.row_rel = c.gAn; p.row_ref = c.An_ref;
-    p.out = c.U; p.b_out = c.zU;
-    if ((rc = launch_pass_tc(STATE, p, dtype, dtype, st)) != MLSTM_OK) return rc;
-    // Inbound states of the blocks and z.  dQ's state step contracts over the value dimension: the pair kernel reads the
-    // states as they are, the one-CTA kernel wants them transposed.
-    const bool pair = chunk_pair_supported(D, dtype, p.chunk_tiles);
-    if ((rc = launch_state_scan(c.U, c.zU, c.An_bound, nullptr, nullptr, pair ? w.statesT : nullptr, c.zstate, nullptr, nullptr, BH,
-                                c.NB, D, dtype, st, nullptr, nullptr, 0, nullptr, pair ? nullptr : w.statesT, 0)) != MLSTM_OK)
-        return rc;
-    // delta = dh . h, n, db -> the backward's per-row vectors (and dh in the input type)
-    if ((rc = launch_bwd_prep(h, dh, b, m, c.gAn, w.gB, w.gBw, w.g, w.dh16, o, d_o, BH, S, Spad, D, h_dtype, dtype, st)) != MLSTM_OK)
-        return rc;
-    const void* dhp = need16 ? w.dh16 : dh;
-    // what every block contributes to the state carried back: P_k = sum_t beta_t q_t dh_t^T (tensor cores), p_k (vector)
-    p.X = q; p.Y = q; p.Z = dhp;
-    p.col_rel = w.gB; p.col_w = w.gBw; p.col_ref = c.An_ref;
-    p.out = c.U; p.b_out = nullptr; p.state_reverse = 1;
-    p.sched_zeroed = 0;     // the second STATE pass of the call: its counter is cleared again by the launcher
-    if ((rc = launch_pass_tc(STATE, p, dtype, dtype, st)) != MLSTM_OK) return rc;
-    p.state_reverse = 0;
-    p.sched_zeroed = 1;
-    {
-        dim3 grid(c.NB, BH);
-        if (dtype == MLSTM_DT_BF16)
-            launch_plain(rvec_partial_kernel<__nv_bfloat16>, grid, dim3(D), 0, st, static_cast<const __nv_bfloat16*>(q), w.gB, c.An_ref,
-                       c.An_bound, w.g, c.zU, S, Spad, c.NB, chunk, D);
-        else
-            launch_plain(rvec_partial_kernel<__half>, grid, dim3(D), 0, st, static_cast<const __half*>(q), w.gB, c.An_ref, c.An_bound, w.g,
-                       c.zU, S, Spad, c.NB, chunk, D);
-        if (cudaGetLastError() != cudaSuccess) return MLSTM_E_CUDA;
-    }
-    // the block recurrence in reverse: R_k [key, value] (for dV and, in the pair kernel, for dK), its transpose (for dK in
-    // the one-CTA kernel) and r_k
-    if ((rc = launch_state_scan(c.U, c.zU, c.An_bound, nullptr, nullptr, c.states, w.rvec, nullptr, nullptr, BH, c.NB, D,
-                                dtype, st, nullptr, nullptr, 0, nullptr, pair ? nullptr : w.statesT2, 1)) != MLSTM_OK)
-        return rc;
-    // dQ = ((dH V^T + g_r) * decay) K within the block, + beta (S_k dh + g z_k) from the inbound state
-    auto pass = [&](int mode) {
-        return pair ? launch_chunk_pair(mode, p, dtype, dtype, st) : launch_pass_tc(mode, p, dtype, dtype, st);
-    };
-    p.X = dhp; p.Y = v; p.Z = k;
-    p.row_rel = w.gB; p.row_ref = c.An_ref; p.row_g = w.g; p.col_rel = c.ga; p.col_w = c.gaw; p.col_ref = c.a_ref; p.col_g = nullptr;
-    p.states = w.statesT; p.zstate = c.zstate;
-    p.out = dq; p.dot_src = q; p.dot_out = w.Rdot;
-    if ((rc = pass(DQC)) != MLSTM_OK) return rc;
-    // dK = ((V dH^T + g_c) * decay) Q within the block, + gamma (R_k v + r_k) from the later blocks
-    p.X = v; p.Y = dhp; p.Z = q;
-    p.row_rel = c.ga; p.row_ref = c.a_ref; p.row_g = nullptr; p.col_rel = w.gB; p.col_w = w.gBw; p.col_ref = c.An_ref; p.col_g = w.g;
-    p.states = pair ? c.states : w.statesT2; p.rvec = w.rvec;
-    p.out = dk; p.dot_src = k; p.dot_out = w.dI;
-    if ((rc = pass(DKC)) != MLSTM_OK) return rc;
-    // dV = ((K Q^T) * decay / n) dH within the block, + gamma R_k^T k from the later blocks
-    p.X = k; p.Y = q; p.Z = dhp;
-    p.col_g = nullptr; p.states = c.states;
-    p.out = dv; p.dot_src = nullptr; p.dot_out = nullptr;
-    if ((rc = pass(DVC)) != MLSTM_OK) return rc;
-    return launch_df(f, w.dI, w.Rdot, df, di, BH, S, Spad, dtype, st, TC_DOT_PARTS, static_cast<long long>(BH) * Spad, c.gscratch);
+    return chunk_bwd_core(dh, q, k, v, f, i, h, m, b, o, d_o, dq, dk, dv, df, di, w, B * NH, S, D, dtype, h_dtype, chunk, 1,
+                          static_cast<cudaStream_t>(stream));
 }
 
 int mlstm_chunk_bwd(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h,
@@ -667,3 +643,57 @@ int mlstm_chunk_sp_apply(const void* q, const void* k, const void* v, const void
 }
 
 }  // extern "C"
+
+namespace mlstm {
+
+// Blocks of 256 positions: at 512 the states cost half, but the passes inside a block wait for their gate warps (16-bit
+// states, B = 16, NH = 8, S = 4096, D = 256, forward + backward: 2.64 ms at 256, 2.91 at 512, 3.31 at 1024).
+constexpr int MM_CHUNK = 256;
+
+// Where the chunkwise form beats the quadratic kernels.  It needs slices (a CTA walks a slice's blocks, 5 us each) and length.
+// Measured bf16, us, quadratic -> chunkwise, forward | backward:
+//   D = 128   BH 32: S 2048 60 -> 70 | 203 -> 190, S 4096 148 -> 121 | 506 -> 338    BH 64: S 1024 44 -> 53 | 150 -> 156,
+//             S 2048 97 -> 88 | 343 -> 267    BH 128: S 1024 72 -> 74 | 250 -> 233, S 4096 596 -> 275 | 2135 -> 904
+//             BH 16: S 4096 83 -> 103 | 274 -> 261, S 8192 258 -> 194 | 878 -> 489
+//   D = 256   BH 32: S 2048 99 -> 101 | 284 -> 295, S 4096 221 -> 203 | 712 -> 569    BH 64: S 1024 78 -> 88 | 237 -> 261,
+//             S 2048 149 -> 148 | 496 -> 458    BH 128: S 1024 139 -> 149 | 456 -> 450, S 4096 986 -> 618 | 3128 -> 1791
+//             BH 16: S 4096 117 -> 140 | 375 -> 381, S 8192 375 -> 317 | 1182 -> 762
+// bf16 only: a state is a sum over positions, and fp16's range (65504) is too small for what the quadratic kernels add up
+// in fp32.  The forced paths keep the kernels they name.
+bool mm_chunk_route(int BH, int S, int D, int dtype, int flags) {
+    if (flags & (MLSTM_F_FORCE_SIMT | MLSTM_F_FORCE_TC)) return false;
+    if (dtype != MLSTM_DT_BF16 || (D != 128 && D != 256)) return false;
+    return S >= 2048 && static_cast<long long>(BH) * S >= 131072;
+}
+
+size_t mm_chunk_fwd_bytes(int BH, int S, int D) { return carve(nullptr, BH, S, D, MM_CHUNK, 2).bytes; }
+
+int mm_chunk_fwd(const void* q, const void* k, const void* v, const void* f, const void* i, void* h, float* m, float* b, void* workspace,
+                 int BH, int S, int D, int dtype, int h_dtype, cudaStream_t st) {
+    ChunkWs w = carve(workspace, BH, S, D, MM_CHUNK, 2);
+    w.m = m;
+    w.b = b;
+    const int Spad = round_up(S, TILE);
+    int rc;
+    // (the gate pass also clears the status word)
+    if ((rc = launch_gates_fwd(f, i, w.ga, w.gAn, w.a_ref, w.An_ref, m, BH, S, Spad, dtype, st, nullptr, nullptr, w.An_bound, MM_CHUNK,
+                               w.gscratch, w.gaw, w.status, STATUS_WORDS)) != MLSTM_OK)
+        return rc;
+    BlockStateArgs a = forward_states(k, v, w, BH, S, Spad, MM_CHUNK);
+    a.U = w.states; a.vec = w.zstate;
+    if ((rc = launch_carried_states(a, D, dtype, st)) != MLSTM_OK) return rc;
+    return launch_fwdc(q, k, v, nullptr, h, h_dtype, w, BH, S, Spad, D, dtype, MM_CHUNK, nullptr, st, 2);
+}
+
+size_t mm_chunk_bwd_bytes(int BH, int S, int D, bool dh_copy) {
+    return carve_bwd_chunk(nullptr, BH, S, D, MM_CHUNK, dh_copy, 2).bytes;
+}
+
+int mm_chunk_bwd(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h, const float* m,
+                 const float* b, const void* o, void* d_o, void* dq, void* dk, void* dv, void* df, void* di, void* workspace, int BH,
+                 int S, int D, int dtype, int h_dtype, cudaStream_t st) {
+    const ChunkBwdWs w = carve_bwd_chunk(workspace, BH, S, D, MM_CHUNK, o || h_dtype != dtype, 2);
+    return chunk_bwd_core(dh, q, k, v, f, i, h, m, b, o, d_o, dq, dk, dv, df, di, w, BH, S, D, dtype, h_dtype, MM_CHUNK, 2, st);
+}
+
+}  // namespace mlstm

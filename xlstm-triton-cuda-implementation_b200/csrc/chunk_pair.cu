@@ -113,6 +113,7 @@ mlstm_chunk_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     const int NP = (NT + 1) / 2;                 // tile pairs per slice
     const int total = NP * p.BH;
     const int npairs = gridDim.x >> 1;
+    const int nparts = p.state_parts == 2 ? 2 : 1;   // 16-bit halves of the carried state
     const bool misaligned = (smem_u32(smem) & 1023u) != 0;   // uniform over the cluster in practice; never seen
 
     struct Item {
@@ -216,9 +217,9 @@ mlstm_chunk_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                         tma_load_3d_pair(dst + c * BOX_BYTES, &tmZ, lead_full, static_cast<int>(rank) * (D / 2) + c * 64,
                                          stream_tile(it, t) * TILE, it.bh);
                 };
-                auto load_state = [&](int u) {   // contraction indices [128 u, 128 u + 128), this CTA's half of the outputs
+                auto load_state = [&](int part, int u) {   // contraction indices [128 u, 128 u + 128), this CTA's half of the outputs
                     if (!open_slot(dst, lead_full)) return;
-                    const int z = it.bh * p.NB + it.blk;
+                    const int z = (it.bh * p.NB + it.blk) * nparts + part;
                     if (STATE_MN) {
                         for (int c = 0; c < D / 128; c++)
                             tma_load_3d_pair(dst + c * BOX_BYTES, &tmS, lead_full, static_cast<int>(rank) * (D / 2) + c * 64, u * 128, z);
@@ -230,7 +231,8 @@ mlstm_chunk_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                 // same order as the MMA issuer consumes
                 load_y(0);
                 if (it.nsteps > 1) load_y(1);
-                for (int u = 0; u < C::NST; u++) load_state(u);
+                for (int part = 0; part < nparts; part++)
+                    for (int u = 0; u < C::NST; u++) load_state(part, u);
                 for (int t = 2; t < it.nsteps && ok; t++) {
                     load_z(t - 2);
                     load_y(t);
@@ -297,28 +299,31 @@ mlstm_chunk_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                     ok = ok && wait_u(bar_accfree, (n & 1) ^ 1);
                     if (!ok) return;
                     tc_fence_after();
+#pragma unroll 1
+                    for (int part = 0; part < nparts; part++) {
 #pragma unroll
-                    for (int u = 0; u < C::NST; u++) {
-                        const int s = slot_it % C::NSLOT;
-                        ok = wait_u(&bar_full[s], (slot_it / C::NSLOT) & 1);
-                        if (!ok) return;
-                        const uint64_t sd = smem_desc_advance(STATE_MN ? mndesc0 : kdesc0, s * C::SLOT_BYTES);
-                        if (issuer) {
+                        for (int u = 0; u < C::NST; u++) {
+                            const int s = slot_it % C::NSLOT;
+                            ok = wait_u(&bar_full[s], (slot_it / C::NSLOT) & 1);
+                            if (!ok) return;
+                            const uint64_t sd = smem_desc_advance(STATE_MN ? mndesc0 : kdesc0, s * C::SLOT_BYTES);
+                            if (issuer) {
 #pragma unroll
-                            for (int kk = 0; kk < 8; kk++) {
-                                const int kx = u * 8 + kk;
-                                mma_ss_pair(car, smem_desc_advance(xdesc, (kx >> 2) * BOX_BYTES + (kx & 3) * 32),
-                                            smem_desc_advance(sd, STATE_MN ? kk * 2048 : (kk >> 2) * (D / 2 * 128) + (kk & 3) * 32),
-                                            idesc_s, kx > 0 ? 1u : 0u);
+                                for (int kk = 0; kk < 8; kk++) {
+                                    const int kx = u * 8 + kk;
+                                    mma_ss_pair(car, smem_desc_advance(xdesc, (kx >> 2) * BOX_BYTES + (kx & 3) * 32),
+                                                smem_desc_advance(sd, STATE_MN ? kk * 2048 : (kk >> 2) * (D / 2 * 128) + (kk & 3) * 32),
+                                                idesc_s, (part > 0 || kx > 0) ? 1u : 0u);
+                                }
+                                if (part == nparts - 1 && u == C::NST - 1) {
+                                    if (!C::SEP) commit_both(bar_st);
+                                    if (it.nsteps <= 2) commit_both(&bar_xfree[xb]);
+                                }
+                                commit_both(&bar_empty[s]);
                             }
-                            if (u == C::NST - 1) {
-                                if (!C::SEP) commit_both(bar_st);
-                                if (it.nsteps <= 2) commit_both(&bar_xfree[xb]);
-                            }
-                            commit_both(&bar_empty[s]);
+                            __syncwarp();
+                            slot_it++;
                         }
-                        __syncwarp();
-                        slot_it++;
                     }
                 };
                 auto second = [&](int u) {  // ACC += W(u) Z(u), both CTAs
@@ -820,7 +825,7 @@ int launch_chunk_pair_one(const PassParams& p, int in_dtype, cudaStream_t st) {
     if ((rc = tc_make_map(&mx, p.X, p.BH, p.S, D, in_dtype, false, 128)) != MLSTM_OK) return rc;
     if ((rc = tc_make_map(&myh, p.Y, p.BH, p.S, D, in_dtype, false, 64)) != MLSTM_OK) return rc;
     if ((rc = tc_make_map(&mz, p.Z, p.BH, p.S, D, in_dtype, false, 128)) != MLSTM_OK) return rc;
-    if ((rc = tc_make_map(&ms, p.states, p.BH * p.NB, D, D, in_dtype, false, STATE_MN ? 128 : D / 2)) != MLSTM_OK) return rc;
+    if ((rc = tc_make_map(&ms, p.states, p.BH * p.NB * (p.state_parts == 2 ? 2 : 1), D, D, in_dtype, false, STATE_MN ? 128 : D / 2)) != MLSTM_OK) return rc;
     auto kern = mlstm_chunk_pair<MODE, D, ABFMT, OutT>;
     {   // the shared-memory opt-in is a per-device property of the kernel: set once per device
         static std::atomic<bool> opted[64];

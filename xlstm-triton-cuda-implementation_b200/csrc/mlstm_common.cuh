@@ -30,14 +30,12 @@
 
 namespace mlstm {
 
-// FWDC and STATE are the two passes of the chunkwise forward (chunk.cu): STATE builds, per block of
-// `chunk_tiles` tiles, U = sum_j w_j k_j v_j^T (rows = key dimensions, X = identity, Y = K, Z = V);
-// FWDC is FWD restricted to the query's own block plus one step that applies the block's inbound
-// state (Y = identity, Z = state), so T = Q and W = Q scaled per row.
-// DQC, DKC, DVC are the backward passes of the chunkwise form: DQ / DK / DV restricted to the row tile's own
-// block plus one step that applies a carried state (the inbound state S_k for dQ; for dK and dV the state
-// R_k = sum over later positions t of exp(A_end(k) - A_t) (scale / n_t) q_t dh_t^T carried BACK over the blocks).
-enum Mode : int { FWD = 0, DQ = 1, DK = 2, DV = 3, FWDC = 4, STATE = 5, DQC = 6, DKC = 7, DVC = 8 };
+// FWDC is the output pass of the chunkwise forward (chunk.cu): FWD restricted to the query's own block plus the block's
+// inbound state.  DQC, DKC, DVC are the backward passes of the chunkwise form: DQ / DK / DV restricted to the row tile's own
+// block plus a carried state (the inbound state S_k for dQ; for dK and dV the state
+// R_k = sum over later positions t of exp(A_end(k) - A_t) (scale / n_t) q_t dh_t^T carried BACK over the blocks).  The
+// states' own pass is chunk_state.cu.  On single CTAs (mm_tc.cu) the state is one more step with Y = identity, Z = state.
+enum Mode : int { FWD = 0, DQ = 1, DK = 2, DV = 3, FWDC = 4, DQC = 6, DKC = 7, DVC = 8 };
 
 constexpr int TILE = 128;      // rows of a tensor-core tile; gate vectors are padded to a multiple of it
 constexpr int REF_BLOCK = 64;  // positions per reference block of the re-centred gate vectors (gates.cu)
@@ -79,11 +77,11 @@ struct PassParams {
     int NB;                  // blocks per slice
     const double* An_bound;  // [BH, NB + 1]  -A*log2e at the block boundaries (entry 0: the inbound carry)
     const void* ident;       // [128, 128] identity in the input type
-    const void* states;      // FWDC and the chunkwise backward passes: [BH, NB, D, D] the state applied to every block
-                             // (input type; rows = the contraction index of the state step)
+    const void* states;      // FWDC and the chunkwise backward passes: [BH, NB, state_parts, D, D] the state applied to every
+                             // block (input type; rows = the contraction index of the state step)
+    int state_parts;         // CTA pairs only: 2 = the state is the sum of two 16-bit halves; else 0 or 1
     const float* zstate;     // FWDC, DQC: [BH, NB, D] inbound normaliser vector of every block
     const float* rvec;       // DKC: [BH, NB, D] vector part of the state carried back from the later blocks
-    int state_reverse;       // STATE: rows carry +A_end(previous block) (contributions to the backward's carried state)
     // FWDC, optional: a carry that became known after the gate pass (sequence-parallel segments).
     // late_bound[bh] = -(A_in + F_in) * log2e, the inbound prefix maximum in this segment's own
     // coordinates; every stabiliser -A*log2e of the slice (rows, block boundaries) becomes
@@ -174,6 +172,21 @@ int launch_gates_fwd(const void* f, const void* i, float* ga_rel, float* gAn_rel
 constexpr int STATUS_WORDS = 64;
 // bytes of `scratch` that let launch_gates_fwd cut long slices into segments (0: not worth it)
 size_t gates_scratch_bytes(int BH, int Spad);
+// states of the chunkwise form (chunk_state.cu, which has the algebra)
+struct BlockStateArgs {
+    const void *X, *Y;       // [BH, S, D]
+    const float* col_w;      // [BH, Spad] exp2 of the column term relative to its reference
+    const double* col_ref;   // [BH, Spad / REF_BLOCK]
+    const float* col_g;      // [BH, Spad] factor of the vector part, or nullptr (1)
+    const double* An_bound;  // [BH, NB + 1]
+    void* U;                 // block_states: [BH, NB, D, D] (rows: X's columns) in the input type; carried_states: [BH, NB, 2, D, D]
+    float* vec;              // [BH, NB, D]
+    int S, Spad, BH, NB, chunk, reverse;
+    int* status;
+};
+// what every block contributes (U, u), resp. the state in front of every block as two 16-bit matrices (hi, mid)
+int launch_block_states(const BlockStateArgs& p, int D, int dtype, cudaStream_t st);
+int launch_carried_states(const BlockStateArgs& p, int D, int dtype, cudaStream_t st);
 // chunk.cu
 int launch_identity(void* ident, int D, int dtype, cudaStream_t st);
 // rec (optional): per-slice records of rec_stride floats that receive S_end | z_end | summary {F, A} (two doubles)
@@ -181,6 +194,17 @@ int launch_state_scan(const void* U, const float* zU, const double* An_bound, co
                       void* states16, float* zstate, float* S_end, float* z_end, int BH, int NB, int D, int dtype,
                       cudaStream_t st, const double* late_bound = nullptr, float* rec = nullptr, size_t rec_stride = 0,
                       const double* summary = nullptr, void* statesT16 = nullptr, int reverse = 0, int* zero_word = nullptr);
+// The parallel entry points' use of the chunkwise form (16-bit inputs, D = 128 or 256, long enough sequences): same
+// results, linear in S.  Nothing that the quadratic kernels keep in fp32 is rounded to 16 bits on the way: the carried
+// states, and what enters them, are held as two 16-bit halves (hi + mid).
+bool mm_chunk_route(int BH, int S, int D, int dtype, int flags);
+size_t mm_chunk_fwd_bytes(int BH, int S, int D);
+int mm_chunk_fwd(const void* q, const void* k, const void* v, const void* f, const void* i, void* h, float* m, float* b, void* workspace,
+                 int BH, int S, int D, int dtype, int h_dtype, cudaStream_t st);
+size_t mm_chunk_bwd_bytes(int BH, int S, int D, bool dh_copy);
+int mm_chunk_bwd(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h, const float* m,
+                 const float* b, const void* o, void* d_o, void* dq, void* dk, void* dv, void* df, void* di, void* workspace, int BH,
+                 int S, int D, int dtype, int h_dtype, cudaStream_t st);
 int launch_bwd_prep(const void* h, const void* dh, const float* b, const float* m, const float* gAn, float* gB,
                     float* gBw, float* g, void* dh_out, const void* o, void* d_o, int BH, int S, int Spad, int D, int h_dtype,
                     int dtype, cudaStream_t st);

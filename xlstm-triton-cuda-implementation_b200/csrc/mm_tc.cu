@@ -130,13 +130,11 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
     constexpr bool IS_DK = (MODE == DK || MODE == DKC);
     // chunkwise passes: the row tile's own block plus one step that applies a carried state
     constexpr bool CHUNKED = (MODE == FWDC || MODE == DQC || MODE == DKC || MODE == DVC);
-    static_assert((!CHUNKED && MODE != STATE) || (ES == 2 && (D == 128 || D == 256)),
+    static_assert(!CHUNKED || (ES == 2 && (D == 128 || D == 256)),
                   "chunkwise passes are built for 16-bit inputs, D = 128 and 256");
     // A carried state is D x D.  As a streamed operand it comes in D / 128 tiles of 128 key rows, each with its own
-    // "state step" (T = the matching 128 columns of the stationary tile through the matching rows of the identity);
-    // as the output of STATE it is written in D / 128 work items of 128 key rows each.
+    // "state step" (T = the matching 128 columns of the stationary tile through the matching rows of the identity).
     constexpr int NS = CHUNKED ? D / TILE : 0;
-    constexpr int NHV = (MODE == STATE) ? D / TILE : 1;
 
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = smem_raw;
@@ -162,17 +160,17 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NBAR);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile int* item_ids = reinterpret_cast<volatile int*>(tmem_slot + 2);  // [4] ring of published work items
-    // [PARTS][NGROUPS][128]: row sums in FWD / STATE, row dots in DQ / DK, one value per gate group and row
+    // [PARTS][NGROUPS][128]: row sums in FWD, row dots in DQ / DK, one value per gate group and row
     float* part_base = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + C::NBAR * 8 + 64);
     constexpr bool STAGED = C::STAGED && !X3;
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int NT = p.Spad / TILE;
-    const int per_slice = (MODE == STATE) ? p.NB * NHV : NT;     // work items per batch*head slice
+    const int per_slice = NT;     // work items per batch*head slice
     const int total = per_slice * p.BH;
 
-    // A work item = one stationary tile (STATE: one block) of one slice.  The CTA is persistent and
+    // A work item = one stationary tile of one slice.  The CTA is persistent and
     // takes the next item from a global counter whenever it is ready for one (the producer thread
     // fetches it and publishes it to the other roles through a four-deep ring in shared memory; it
     // can run at most two items ahead of the slowest role, see the waits on bar_xfree / bar_accfree).
@@ -183,7 +181,7 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         return ok ? __shfl_sync(0xffffffffu, item_ids[n & 3], 0) : -1;
     };
     struct Item {
-        int bh, tile, blk, first, nsteps, half;
+        int bh, tile, blk, first, nsteps;
     };
     auto decode = [&](int id) {
         Item it;
@@ -195,24 +193,20 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         const int set_size = min(SLICE_SET, p.BH - set * SLICE_SET);
         const int w = within / set_size;
         it.bh = set * SLICE_SET + (within - w * set_size);
-        // tile: the stationary tile (STATE: the block).  nsteps / stream_tile: what is streamed.
+        // tile: the stationary tile.  nsteps / stream_tile: what is streamed.
         //   FWD, DQ   key tiles 0..tile, diagonal last          DK, DV  query tiles tile..NT-1, diagonal first
         //   FWDC, DQC the first NS steps apply the block's inbound state, then key tiles block_start..tile
         //   DKC, DVC  the first NS steps apply the state carried back from the later blocks, then query tiles tile..block_end
-        //   STATE     the block's tiles
-        it.tile = (MODE == STATE) ? w / NHV : (ROWS_ARE_Q ? (NT - 1 - w) : w);
-        it.half = (MODE == STATE) ? w % NHV : 0;     // STATE: which 128 key rows of the block's state
-        it.blk = CHUNKED ? it.tile / p.chunk_tiles : (MODE == STATE ? it.tile : 0);
-        it.first = (CHUNKED || MODE == STATE) ? it.blk * p.chunk_tiles : 0;
+        it.tile = ROWS_ARE_Q ? (NT - 1 - w) : w;
+        it.blk = CHUNKED ? it.tile / p.chunk_tiles : 0;
+        it.first = CHUNKED ? it.blk * p.chunk_tiles : 0;
         const int last = min(it.first + p.chunk_tiles, NT) - 1;   // last tile of the block
         it.nsteps = CHUNKED ? (ROWS_ARE_Q ? (it.tile - it.first + 1 + NS) : (last - it.tile + 1 + NS))
-                  : (MODE == STATE) ? (min(p.chunk_tiles, NT - it.first))
                   : (ROWS_ARE_Q ? (it.tile + 1) : (NT - it.tile));
         return it;
     };
     auto stream_tile = [&](const Item& it, int t) {
         if (CHUNKED) return ROWS_ARE_Q ? (it.first + t - NS) : (it.tile + t - NS);  // t >= NS
-        if (MODE == STATE) return it.first + t;
         return ROWS_ARE_Q ? t : (it.tile + t);
     };
     auto is_state_step = [&](int t) { return CHUNKED && t < NS; };
@@ -289,8 +283,7 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
                 if (!ok) break;
                 mbar_expect_tx(bar_x, C::X_BYTES);
                 for (int c = 0; c < DL / C::EPB; c++) {
-                    if (MODE == STATE) tma_load_3d(sX + c * BOX_BYTES, &tmI, bar_x, c * C::EPB, it.half * TILE, 0);
-                    else tma_load_3d(sX + c * BOX_BYTES, &tmX, bar_x, c * C::EPB, it.tile * TILE, it.bh);
+                    tma_load_3d(sX + c * BOX_BYTES, &tmX, bar_x, c * C::EPB, it.tile * TILE, it.bh);
                 }
                 auto load_y = [&](int t) {
                     if (is_state_step(t)) load_tile(&tmI, 0, t * TILE, 0);
@@ -512,7 +505,7 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         [[maybe_unused]] uint8_t* stage = sOut + (warp - 2) * C::STAGE_BYTES;
         if (STAGED && lane == 0) prefetch_tmap(&tmO);
         // Row terms of a work item: the row part of the exponent in double (the column block's reference is added
-        // per block; STATE: rows are key dimensions and every row carries the block-end stabiliser), the weight of
+        // per column block), the weight of
         // the inbound-state step of FWDC (exp(A_prev_block_end - A_row) / sqrt(D); -inf when there is no carry)
         // and the additive term of DQ.  Fetching (the loads) and combining (the first use of what was loaded) are
         // separate steps: the next item's terms are requested before the accumulator wait of this item and combined
@@ -525,16 +518,14 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
             RowRaw rr{0.0f, 0.0f, 0.0, 0.0, 0.0, static_cast<double>(INFINITY)};
             const int grow = it.tile * TILE + r;
             const size_t vec_base = static_cast<size_t>(it.bh) * p.Spad;
-            if (CHUNKED || MODE == STATE) {
+            if (CHUNKED) {
                 const double* bound = p.An_bound + static_cast<size_t>(it.bh) * (p.NB + 1) + it.blk;
                 rr.b0 = bound[0];
                 rr.b1 = bound[1];
                 if (MODE == FWDC && p.late_bound) rr.lb = p.late_bound[it.bh];
             }
-            if (MODE != STATE) {
-                rr.rel = p.row_rel[vec_base + grow];
-                rr.ref = p.row_ref[static_cast<size_t>(it.bh) * (p.Spad / REF_BLOCK) + grow / REF_BLOCK];
-            }
+            rr.rel = p.row_rel[vec_base + grow];
+            rr.ref = p.row_ref[static_cast<size_t>(it.bh) * (p.Spad / REF_BLOCK) + grow / REF_BLOCK];
             if (IS_DQ) rr.g = p.row_g[vec_base + grow];
             return rr;
         };
@@ -554,9 +545,7 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         const double negA = static_cast<double>(raw.rel) + raw.ref;
         const double negA_c = (MODE == FWDC) ? fmin(negA, raw.lb) : negA;
         const float m_shift = (MODE == FWDC) ? static_cast<float>((negA - negA_c) * 0.6931471805599453) : 0.0f;
-        // STATE: every row carries the block's stabiliser: -A_end(block) for the forward states, +A_end(previous
-        // block) for the states carried back in the backward (weights exp(A_end(k-1) - A_t) scale / n_t)
-        const double er_d = (MODE == STATE) ? (p.state_reverse ? -raw.b0 : raw.b1) : negA_c + static_cast<double>(p.er_add);
+        const double er_d = negA_c + static_cast<double>(p.er_add);
         // log2 of the row weight of the state step: FWDC, DQC exp(A_end(k-1) - A_t) (times scale, resp. scale / n_t);
         // DKC, DVC exp(a_j - A_end(k))
         const float er_state = !CHUNKED ? 0.0f
@@ -570,7 +559,7 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
             const int buf = gt & 1;
             const bool state_step = is_state_step(t);
             const int st = state_step ? 0 : stream_tile(it, t);
-            const bool diag = (MODE != STATE) && !state_step && (st == tile);
+            const bool diag = !state_step && (st == tile);
             // On the diagonal tile the 32 x 32 patch of a gate group and a row quarter lies wholly on the masked side
             // for six of the sixteen (group, quarter) pairs: those warps write zeros over their part of T and read nothing.
             if (diag && (ROWS_ARE_Q ? (grp > (warp & 3)) : (grp < (warp & 3)))) {
@@ -653,7 +642,7 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
                 for (int j = 0; j < 32; j++) {
                     const float tu = IS_DQ ? fmaf(__uint_as_float(tv[j]), u, gu) : __uint_as_float(tv[j]) * u;
                     const float wj = tu * cv[j];
-                    if (IS_FWD || MODE == STATE) rowsum += wj;
+                    if (IS_FWD) rowsum += wj;
                     cv[j] = wj;
                 }
             }
@@ -698,7 +687,7 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         constexpr int CW = QUART < 32 ? QUART : 32;    // columns per TMEM load
         constexpr int VEC = 16 / sizeof(SideT);        // elements per 16-byte access of the tensors read in the epilogue
         const int c0 = grp * QUART;
-        const bool row_ok = (MODE == STATE) ? true : (grow < p.S);
+        const bool row_ok = grow < p.S;
         float* part = part_base + (C::PARTS == 2 ? (n & 1) * NGROUPS * 128 : 0);
         float inv_n = 1.0f;
         auto exchange = [&](float x) {   // sum of one value per gate group for this row (once per item)
@@ -709,10 +698,6 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
             return ok ? (part[r] + part[128 + r]) + (part[256 + r] + part[384 + r]) : 0.0f;
         };
         auto row_sums = [&]() {
-            if (MODE == STATE) {
-                const float zsum = exchange(rowsum);
-                if (ok && grp == 0 && p.b_out) p.b_out[(static_cast<size_t>(bh) * p.NB + blk) * D + it.half * TILE + r] = zsum;
-            }
             if (IS_FWD) {
                 // on its way during the exchange
                 const float mrow = row_ok ? p.m[static_cast<size_t>(bh) * p.S + grow] + m_shift : 0.0f;
@@ -748,10 +733,7 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
             tc_fence_after();
             if (!sums_early) row_sums();
             if (!ok) break;
-            // STATE writes block (bh, blk) of [BH, NB, D, D]; everything else row `grow` of [BH, S, D]
-            const size_t row_off = (MODE == STATE)
-                                       ? ((static_cast<size_t>(bh) * p.NB + blk) * D + it.half * TILE + r) * D
-                                       : (static_cast<size_t>(bh) * p.S + (row_ok ? grow : 0)) * D;
+            const size_t row_off = (static_cast<size_t>(bh) * p.S + (row_ok ? grow : 0)) * D;
             float dot = 0.0f;
             OutT* orow = reinterpret_cast<OutT*>(p.out) + row_off + c0;
             const SideT* ogate_row = (IS_FWD && p.ogate) ? reinterpret_cast<const SideT*>(p.ogate) + row_off + c0 : nullptr;
@@ -845,8 +827,7 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
                         __syncwarp();
                         if (lane == 0) {
                             const int x = c0 + ch * 32 + sub * (64 / static_cast<int>(sizeof(OutT)));
-                            if (MODE == STATE) tma_store_3d(&tmO, stage, x, (warp & 3) * 32, bh * p.NB + blk);
-                            else tma_store_3d(&tmO, stage, x, tile * TILE + (warp & 3) * 32, bh);
+                            tma_store_3d(&tmO, stage, x, tile * TILE + (warp & 3) * 32, bh);
                             bulk_commit();
                         }
                     }
@@ -1007,7 +988,7 @@ int launch_one(const PassParams& p_in, int in_dtype, cudaStream_t st) {
     mi = mx;
     ms = mx;
     constexpr bool CHUNKED = (MODE == FWDC || MODE == DQC || MODE == DKC || MODE == DVC);
-    if (CHUNKED || MODE == STATE) {
+    if (CHUNKED) {
         if (!p.ident || p.chunk_tiles <= 0 || p.NB <= 0 || !p.An_bound) return MLSTM_E_ARG;
         if ((rc = make_map(&mi, p.ident, 1, D, D, in_dtype)) != MLSTM_OK) return rc;
     }
@@ -1018,8 +999,7 @@ int launch_one(const PassParams& p_in, int in_dtype, cudaStream_t st) {
     mo = mx;
     if (TcCfg<DL, ABFMT == 2 ? 4 : 2>::STAGED && !X3) {
         constexpr int out_dtype = sizeof(OutT) == 4 ? MLSTM_DT_F32 : (ABFMT == 1 ? MLSTM_DT_BF16 : MLSTM_DT_F16);
-        if (MODE == STATE) rc = tc_make_map_out(&mo, p.out, p.BH * p.NB, D, D, out_dtype, 32);
-        else rc = tc_make_map_out(&mo, p.out, p.BH, p.S, D, out_dtype, 32);
+        rc = tc_make_map_out(&mo, p.out, p.BH, p.S, D, out_dtype, 32);
         if (rc != MLSTM_OK) return rc;
     }
     auto kern = mlstm_tc_pass<MODE, D, ABFMT, OutT, X3>;
@@ -1039,7 +1019,7 @@ int launch_one(const PassParams& p_in, int in_dtype, cudaStream_t st) {
         }
     }
     const int NT = p.Spad / TILE;
-    const long long total = static_cast<long long>(MODE == STATE ? p.NB * (D / TILE) : NT) * p.BH;
+    const long long total = static_cast<long long>(NT) * p.BH;
     if (total > 0x7fffffffLL) return MLSTM_E_SHAPE;
     const int sms = sm_count();
     if (sms <= 0) return MLSTM_E_CUDA;
@@ -1169,10 +1149,6 @@ int launch_pass_tc(int mode, const PassParams& p, int in_dtype, int out_dtype, c
             if (p.D == 256) return launch_fmt<FWDC, 256>(p, in_dtype, out_dtype, st);
             if (p.D != 128) return MLSTM_E_UNSUPPORTED;
             return launch_fmt<FWDC, 128>(p, in_dtype, out_dtype, st);
-        case STATE:
-            if (p.D == 256) return launch_fmt<STATE, 256>(p, in_dtype, out_dtype, st);
-            if (p.D != 128) return MLSTM_E_UNSUPPORTED;
-            return launch_fmt<STATE, 128>(p, in_dtype, out_dtype, st);
         case DQC:
             if (p.D == 256) return launch_fmt<DQC, 256>(p, in_dtype, out_dtype, st);
             if (p.D != 128) return MLSTM_E_UNSUPPORTED;
