@@ -388,3 +388,33 @@ def test_long_sequences_take_the_chunkwise_form(gc, BH, S, D, gated, pad):
             refs.append(y["dh"].double() * ref * sg * (1.0 + y["o"].double() * (1.0 - sg)))
         for name, a, a2, r in zip(("dq", "dk", "dv", "df", "di", "do"), gr, gr2, refs):
             assert err(cut(a), r) < 1.25 * err(cut(a2), r), name
+
+
+@pytest.mark.parametrize("B,NH,S,D,dtype", [
+    (1, 2, 64, 8, torch.float32),          # one tile
+    (2, 1, 65, 32, torch.float32),         # a tile and one row
+    (1, 3, 200, 72, torch.float32),        # a partial column tile
+    (1, 2, 321, 256, torch.float32),
+    (1, 2, 130, 96, torch.float16),
+    (1, 2, 8190, 8, torch.float32),        # the longest: slices in groups of one
+])
+def test_cuda_core_arithmetic_in_two_stages(gc, B, NH, S, D, dtype):
+    """Head dimensions outside the tensor-core set: against the one-stage kernel (the same fp32 products, added up in another
+    order: sums of S terms, S * 2^-24 of the largest at worst) and, where it is quick, the oracle."""
+    x = gc.make_inputs(B, NH, S, D, dtype, f_mean=1.0, qkv_scale=D ** -0.5, seed=S + D, with_o=True)
+    h, m, b = gc.run_forward(x)
+    h1, m1, b1 = gc.run_forward(x, flags=gc._lib.F_FORCE_SIMT)
+    tol = TOL_F32 if dtype == torch.float32 else 1e-3     # 16 bits: the gradients are rounded to 2^-11
+    assert orc.max_abs_rel(h, h1.cpu()) < TOL_F32
+    assert orc.max_abs_rel(b, b1.cpu()) < TOL_F32
+    assert torch.equal(m, m1)
+    g, g1 = gc.run_backward(x, h, m, b), gc.run_backward(x, h1, m1, b1, flags=gc._lib.F_FORCE_SIMT)
+    for name, a, r in zip(("dq", "dk", "dv", "df", "di"), g, g1):
+        assert orc.max_abs_rel(a, r.cpu()) < 3 * tol, name
+    o = x["o"].cuda()
+    scan = gc.PKG.mlstm_scan(*(x[n].cuda() for n in ("q", "k", "v", "f", "i")), o, 1, 1, allow_tf32=False)
+    assert orc.max_abs_rel(scan, (h * torch.nn.functional.silu(o.float())).cpu()) < tol
+    if S <= 400:
+        assert orc.max_abs_rel(h, gc.oracle_forward(x)[0]) < TOL_F32
+        for name, a, r in zip(("dq", "dk", "dv", "df", "di"), g, gc.oracle_backward(x, torch.float32)):
+            assert orc.max_abs_rel(a, r) < 3 * tol, name

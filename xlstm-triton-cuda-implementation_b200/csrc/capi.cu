@@ -161,6 +161,21 @@ int round_inputs(const void** ptrs, int count, void* buf, int BH, int S, int D, 
     return MLSTM_OK;
 }
 
+// The CUDA-core arithmetic in two stages (simt_gemm.cu), where the caller's workspace has room for S x S matrices;
+// MLSTM_F_FORCE_SIMT and MLSTM_F_NO_SPLIT keep the one-stage kernel, which is the cross-check of everything else.
+bool simt_two_stage(int S, int D, int dtype, int flags) {
+    int rc;
+    return !(flags & (MLSTM_F_FORCE_SIMT | MLSTM_F_NO_SPLIT)) && pass_kind(S, D, dtype, flags, &rc) == KIND_SIMT && simt_gemm_supported(S);
+}
+// scratch of forward_impl behind the gate vectors: converted operands, or the two-stage form's matrices
+size_t fwd_extra_bytes(int BH, int S, int D, int dtype, int flags) {
+    return simt_two_stage(S, D, dtype, flags) ? simt_gemm_fwd_bytes(BH, S) : tf32_copy_bytes(BH, S, D, dtype, flags, 3);
+}
+size_t simt_bwd_extra_bytes(int BH, int S, int D) {
+    const size_t vec = static_cast<size_t>(BH) * round_up(S, TILE) * sizeof(float);
+    return 2 * al(simt_gemm_matrix_bytes(BH, S)) + 2 * al(vec * ((D + 63) / 64));
+}
+
 int run_pass(int kind, int mode, const PassParams& p, int in_dt, int out_dt, cudaStream_t st) {
     if (kind == KIND_TC_X3) return launch_pass_tc_x3(mode, p, st);
     return kind == KIND_TC ? launch_pass_tc(mode, p, in_dt, out_dt, st) : launch_pass_simt(mode, p, in_dt, out_dt, st);
@@ -168,7 +183,7 @@ int run_pass(int kind, int mode, const PassParams& p, int in_dt, int out_dt, cud
 
 int forward_impl(const void* q, const void* k, const void* v, const void* f, const void* i, const void* o, void* h,
                  float* m, float* b, const FwdWs& w, int BH, int S, int D, int dtype, int h_dtype, int flags,
-                 cudaStream_t st, void* tf32buf = nullptr) {
+                 cudaStream_t st, void* extra = nullptr) {
     int rc;
     const int kind = pass_kind(S, D, dtype, flags, &rc);
     if (rc != MLSTM_OK) return rc;
@@ -177,10 +192,14 @@ int forward_impl(const void* q, const void* k, const void* v, const void* f, con
     if ((rc = launch_gates_fwd(f, i, w.ga, w.gAn, w.a_ref, w.An_ref, m, BH, S, Spad, dtype, st, nullptr, nullptr, nullptr, 0, nullptr,
                                w.gaw, w.status, STATUS_WORDS)) != MLSTM_OK)
         return rc;
+    if (extra && simt_two_stage(S, D, dtype, flags)) {
+        SimtGemmArgs a{S, Spad, BH, D, w.ga, w.gAn, w.a_ref, w.An_ref, m, b, static_cast<float*>(extra)};
+        return launch_simt_gemm_fwd(a, q, k, v, o, h, dtype, h_dtype, st);
+    }
     const void* in[3] = {q, k, v};
     if (kind != KIND_SIMT && dtype == MLSTM_DT_F32) {
-        if (!tf32buf) return MLSTM_E_WORKSPACE;
-        if ((rc = round_inputs(in, 3, tf32buf, BH, S, D, kind, st)) != MLSTM_OK) return rc;
+        if (!extra) return MLSTM_E_WORKSPACE;
+        if ((rc = round_inputs(in, 3, extra, BH, S, D, kind, st)) != MLSTM_OK) return rc;
     }
     PassParams p{};
     p.S = S; p.Spad = Spad; p.BH = BH; p.D = D;
@@ -282,7 +301,7 @@ size_t mlstm_mm_fwd_workspace(int B, int NH, int S, int D, int dtype, int flags)
     if (mm_fwd_two_pass(S, D, dtype, MLSTM_DT_F32, flags))
         return carve_fwd(nullptr, B * NH, S, false).bytes + two_pass_extra_bytes(B * NH, S, dtype);
     if (mm_chunk_route(B * NH, S, D, dtype, flags)) return mm_chunk_fwd_bytes(B * NH, S, D);
-    return carve_fwd(nullptr, B * NH, S, false).bytes + tf32_copy_bytes(B * NH, S, D, dtype, flags, 3);
+    return carve_fwd(nullptr, B * NH, S, false).bytes + fwd_extra_bytes(B * NH, S, D, dtype, flags);
 }
 
 int mlstm_mm_fwd(const void* q, const void* k, const void* v, const void* f, const void* i, void* h, float* m, float* b,
@@ -304,7 +323,7 @@ int mlstm_mm_fwd(const void* q, const void* k, const void* v, const void* f, con
         if (!workspace || workspace_bytes < mm_chunk_fwd_bytes(B * NH, S, D) || !aligned16(workspace)) return MLSTM_E_WORKSPACE;
         return mm_chunk_fwd(q, k, v, f, i, h, m, b, workspace, B * NH, S, D, dtype, h_dtype, static_cast<cudaStream_t>(stream));
     }
-    const size_t extra = tf32_copy_bytes(B * NH, S, D, dtype, flags, 3);
+    const size_t extra = fwd_extra_bytes(B * NH, S, D, dtype, flags);
     if (!workspace || workspace_bytes < w.bytes + extra || !aligned16(workspace)) return MLSTM_E_WORKSPACE;
     return forward_impl(q, k, v, f, i, nullptr, h, m, b, w, B * NH, S, D, dtype, h_dtype, flags,
                         static_cast<cudaStream_t>(stream), extra ? static_cast<uint8_t*>(workspace) + w.bytes : nullptr);
@@ -322,6 +341,7 @@ static size_t mm_bwd_workspace(int B, int NH, int S, int D, int dtype, int h_dty
     if (mm_chunk_route(B * NH, S, D, dtype, flags)) return mm_chunk_bwd_bytes(B * NH, S, D, dh_copy_bytes(dtype, h_dtype, gated) != 0);
     const size_t own = carve_bwd(nullptr, B * NH, S, D, dh_copy_bytes(dtype, h_dtype, gated)).bytes;
     if (mm_bwd_two_pass(S, D, dtype, flags)) return own + two_pass_bwd_extra_bytes(B * NH, S, D, dtype);
+    if (simt_two_stage(S, D, dtype, flags)) return own + simt_bwd_extra_bytes(B * NH, S, D);
     return own + tf32_copy_bytes(B * NH, S, D, dtype, flags, 4);
 }
 
@@ -377,7 +397,8 @@ static int mm_bwd_impl(const void* dh, const void* q, const void* k, const void*
         if ((rc = launch_scan_gemm_bwd(a, dtype, st)) != MLSTM_OK) return rc;
         return launch_df(f, a.dI, a.R, df, di, BH, S, Spad, dtype, st, D / 256, a.dot_stride);
     }
-    const size_t extra = tf32_copy_bytes(BH, S, D, dtype, flags, 4);
+    const bool two_stage = simt_two_stage(S, D, dtype, flags);
+    const size_t extra = two_stage ? simt_bwd_extra_bytes(BH, S, D) : tf32_copy_bytes(BH, S, D, dtype, flags, 4);
     if (!workspace || workspace_bytes < w.bytes + extra || !aligned16(workspace)) return MLSTM_E_WORKSPACE;
     const int kind = pass_kind(S, D, dtype, flags, &rc);
     if (rc != MLSTM_OK) return rc;
@@ -388,6 +409,16 @@ static int mm_bwd_impl(const void* dh, const void* q, const void* k, const void*
     if ((rc = launch_bwd_prep(h, dh, b, m, w.gAn, w.gB, w.gBw, w.g, w.dh16, o, d_o, BH, S, Spad, D, h_dtype, dtype, st)) != MLSTM_OK)
         return rc;
     const void* dhp = dh_es ? w.dh16 : dh;  // dh in the element type of q, k, v
+    if (two_stage) {
+        uint8_t* base = static_cast<uint8_t*>(workspace) + w.bytes;
+        const size_t mat = al(simt_gemm_matrix_bytes(BH, S)), vec = static_cast<size_t>(BH) * Spad * sizeof(float);
+        const int nparts = (D + 63) / 64;
+        SimtGemmArgs a{S, Spad, BH, D, w.ga, w.gAn, w.a_ref, w.An_ref, nullptr, nullptr, reinterpret_cast<float*>(base)};
+        SimtGemmBwdArgs g{q, k, v, dhp, dq, dk, dv, w.gB, w.g, reinterpret_cast<float*>(base + mat), reinterpret_cast<float*>(base + 2 * mat),
+                          reinterpret_cast<float*>(base + 2 * mat + al(vec * nparts)), static_cast<long long>(BH) * Spad};
+        if ((rc = launch_simt_gemm_bwd(a, g, dtype, st)) != MLSTM_OK) return rc;
+        return launch_df(f, g.dI, g.R, df, di, BH, S, Spad, dtype, st, nparts, g.dot_stride);
+    }
     const void* orig_q = q;
     const void* orig_k = k;
     if (kind != KIND_SIMT && dtype == MLSTM_DT_F32) {  // converted copies of q, k, v, dh
@@ -460,7 +491,7 @@ size_t mlstm_scan_fwd_workspace(int B, int NH, int S, int D, int dtype, int flag
         case SCAN_TWO_PASS:
             return carve_fwd(nullptr, B * NH, S, true).bytes + two_pass_extra_bytes(B * NH, S, dtype);
         case SCAN_CHUNKWISE: return mlstm_chunk_workspace(B, NH, S, D, dtype, SCAN_CHUNK);
-        default: return carve_fwd(nullptr, B * NH, S, true).bytes + tf32_copy_bytes(B * NH, S, D, dtype, flags, 3);
+        default: return carve_fwd(nullptr, B * NH, S, true).bytes + fwd_extra_bytes(B * NH, S, D, dtype, flags);
     }
 }
 
@@ -489,7 +520,7 @@ int mlstm_scan_fwd(const void* q, const void* k, const void* v, const void* f, c
         return two_pass_forward(q, k, v, f, i, o, static_cast<float*>(h), w.m, nullptr, w, static_cast<uint8_t*>(workspace) + w.bytes,
                                 BH, S, D, dtype, st);
     if ((flags & MLSTM_F_FORCE_TC) && D > 256) return MLSTM_E_UNSUPPORTED;
-    const size_t extra = tf32_copy_bytes(BH, S, D, dtype, flags, 3);
+    const size_t extra = fwd_extra_bytes(BH, S, D, dtype, flags);
     void* tf32buf = extra ? static_cast<uint8_t*>(workspace) + w.bytes : nullptr;
     return forward_impl(q, k, v, f, i, o, h, w.m, w.b, w, BH, S, D, dtype, MLSTM_DT_F32, flags, st, tf32buf);
 }

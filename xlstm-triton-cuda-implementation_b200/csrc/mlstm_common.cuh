@@ -214,6 +214,31 @@ int launch_df(const void* f, const float* dI, const float* R, void* df, void* di
               cudaStream_t st, int nparts = 1, long long part_stride = 0, double* scratch = nullptr);
 constexpr int TC_DOT_PARTS = 4;   // gate groups of the tensor-core passes
 int launch_pass_simt(int mode, const PassParams& p, int in_dtype, int out_dtype, cudaStream_t st);
+// fp32 FMA in two stages with S x S matrices in scratch (simt_gemm.cu).  Gate vectors of launch_gates_fwd and launch_bwd_prep
+// for all BH slices.  W0, W1: simt_gemm_matrix_bytes each (forward: one, simt_gemm_fwd_bytes with the row-sum partials
+// behind it); R, dI: [D / 64 rounded up][BH, Spad] partial row dots, dot_stride apart, for launch_df
+struct SimtGemmArgs {
+    int S, Spad, BH, D;
+    const float *ga, *gAn;
+    const double *a_ref, *An_ref;
+    const float* m;
+    float* b;
+    float* W0;
+};
+struct SimtGemmBwdArgs {
+    const void *q, *k, *v, *dh;
+    void *dq, *dk, *dv;
+    const float *gB, *g;
+    float *W1, *R, *dI;
+    long long dot_stride;
+};
+bool simt_gemm_supported(int S);
+int simt_gemm_group(int BH, int S);    // slices whose matrices are in scratch at one time
+size_t simt_gemm_fwd_bytes(int BH, int S);
+size_t simt_gemm_matrix_bytes(int BH, int S);
+int launch_simt_gemm_fwd(const SimtGemmArgs& a, const void* q, const void* k, const void* v, const void* o, void* h, int dtype,
+                         int h_dtype, cudaStream_t st);
+int launch_simt_gemm_bwd(const SimtGemmArgs& a, const SimtGemmBwdArgs& b, int dtype, cudaStream_t st);
 int launch_pass_tc(int mode, const PassParams& p, int in_dtype, int out_dtype, cudaStream_t st);
 bool tc_supported(int S, int D, int in_dtype);
 // chunkwise output and backward passes on CTA pairs (chunk_pair.cu); states: one row-major copy [key, value] for all modes
