@@ -46,6 +46,18 @@ def algorithmic_flops(B, NH, S, D):
     return 4 * D * pairs * B * NH, 10 * D * pairs * B * NH
 
 
+def carried_flops(B, NH, S, D, block=256):
+    """The same per position when the sequence is taken in blocks with a carried state (what the library does with long
+    bf16 sequences of many slices): the part inside the block, and the state's update and use."""
+    fwd = B * NH * S * (4 * D * (block + 1) / 2 + 4 * D * D)
+    return fwd, 2.5 * fwd
+
+
+def takes_carried_form(slices, S):
+    """Whether the parallel entry points take the chunkwise form for the headline's D and type (mm_chunk_route, csrc/chunk.cu)."""
+    return S >= 2048 and slices * S >= 131072
+
+
 def measured_peaks():
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(path):
@@ -720,7 +732,7 @@ def main():
         for x in t.values():
             x.grad = None
         del t, dh32
-        ff, fb = algorithmic_flops(B, NH, S, D)
+        ff, fb = (carried_flops if takes_carried_form(n_local, S) else algorithmic_flops)(B, NH, S, D)
         secondary["cfg4_dropin"] = {
             "workload": "the headline step through Triton_mLSTM.apply(q,k,v,f,i,SB,NUM_WARPS) + h.backward(dh): fp32 h and dh",
             "ms": ms_dropin, "value": B * S / (ms_dropin * 1e-3), "unit": "tokens/s",
@@ -769,12 +781,16 @@ def main():
         ms_per_step = elapsed_ms / args.steps
         value = tokens_per_step / (ms_per_step * 1e-3)
         e2e_value = tokens_per_step / (e2e_ms / e2e_steps * 1e-3)
-        ff, fb = algorithmic_flops(B, NH, S, D)
-        roof = roofline_tensor(ctx, (ff + fb) / world, fwd_ms + bwd_ms, clocks, elapsed_ms * 1e-3)
+        carried = takes_carried_form(n_local, S)
+        ff, fb = (carried_flops if carried else algorithmic_flops)(B, NH, S, D)
+        if carried:
+            # bytes the step cannot do without, 16 bits each: q, k, v in and h out; dh, q, k, v, h in and dq, dk, dv out
+            roof = roofline_hbm(ctx, 24.0 * n_local * S * D, fwd_ms + bwd_ms)
+            roof["kernel"] = "states_kernel, mlstm_chunk_pair (FWDC, DQC, DKC, DVC) and the gate passes of one step, per GPU"
+        else:
+            roof = roofline_tensor(ctx, (ff + fb) / world, fwd_ms + bwd_ms, clocks, elapsed_ms * 1e-3)
+            roof["kernel"] = "mlstm_tc_pass_pair (FWD, DQ, DK, DV launches of one step, with the gate passes), per GPU"
         roof.update({
-            "kernel": "mlstm_tc_pass_pair (FWD, DQ, DK, DV launches of one step, with the gate passes), per GPU",
-            # DRAM bytes per launch from the ncu capture in profiles/ (B=4 case, scaled by slices)
-            "traffic": 1.18e9 / world, "traffic_source": "ncu, B=4 case scaled by slices, average of the four passes",
             "fwd_tflops": ff / world / (fwd_ms * 1e-3) / 1e12, "bwd_tflops": fb / world / (bwd_ms * 1e-3) / 1e12,
             "fwd_ms": fwd_ms, "bwd_ms": bwd_ms, "timed_region_s": elapsed_ms * 1e-3,
             "ms_times_mhz": (fwd_ms + bwd_ms) * clocks["sm_mhz"] if clocks.get("sm_mhz") else None})
@@ -788,7 +804,7 @@ def main():
             "e2e": {"value": e2e_value, "unit": "tokens/s", "h2d_bytes_per_step": h2d_all, "d2h_bytes_per_step": d2h_all,
                     "ms_per_step": e2e_ms / e2e_steps,
                     "pipeline": "3 streams per rank: H2D of step s+1, compute of step s and D2H of step s-1 overlap; bytes summed over ranks"},
-            "gpu_launches": 8 * args.steps,
+            "gpu_launches": (11 if takes_carried_form(n_local, S) else 8) * args.steps,
             "clocks": clocks,
         }
         if secondary:
