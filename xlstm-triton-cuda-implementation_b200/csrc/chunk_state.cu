@@ -22,7 +22,8 @@
 // S = 4096, D = 256, carried: 128 us; now 100, 5.4 TB/s).  The D / 128 row halves of a slice run on neighbouring CTAs and
 // share Y in L2.  Slots of 64 positions.  With few slices it is latency, 5 us per block of 256 (BH = 32, D = 128): see the
 // rule in chunk.cu for where the carried form is used.  block_states took the place of a pass that brought K through an
-// identity into TMEM to transpose it (S = 65536, NH = 8, D = 128: forward a call 325 -> 301 us together with the output pass on pairs; S = 16384, training step: 477 -> 462).
+// identity into TMEM to transpose it (S = 65536, NH = 8, D = 128: forward 325 -> 301 us together with the output pass on
+// pairs; S = 16384, training step: 477 -> 462).
 #include <atomic>
 
 #include "mlstm_common.cuh"

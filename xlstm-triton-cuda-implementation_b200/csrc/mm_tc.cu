@@ -505,9 +505,8 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         [[maybe_unused]] uint8_t* stage = sOut + (warp - 2) * C::STAGE_BYTES;
         if (STAGED && lane == 0) prefetch_tmap(&tmO);
         // Row terms of a work item: the row part of the exponent in double (the column block's reference is added
-        // per column block), the weight of
-        // the inbound-state step of FWDC (exp(A_prev_block_end - A_row) / sqrt(D); -inf when there is no carry)
-        // and the additive term of DQ.  Fetching (the loads) and combining (the first use of what was loaded) are
+        // per column block), the weight of the inbound-state step of FWDC (exp(A_prev_block_end - A_row) / sqrt(D); -inf when
+        // there is no carry) and the additive term of DQ.  Fetching (the loads) and combining (the first use of what was loaded) are
         // separate steps: the next item's terms are requested before the accumulator wait of this item and combined
         // only when that item starts, so nobody waits for those loads.
         struct RowRaw {

@@ -18,6 +18,9 @@ fp32 dot products on the CUDA cores.  Setting the environment variable ``MLSTM_B
 ``flags=_lib.F_ALLOW_TF32`` to the two plain functions) trades accuracy for speed: single tf32 products
 (D in {64, 128, 256}; error about 5e-4).  ``fp32_math_mode(D)`` says which of these a call will use.
 
+Long bfloat16 sequences of many slices (D = 128 or 256, S >= 2048, B * NH * S >= 131072) are taken in blocks of 256 with
+a carried state (linear in S instead of quadratic; the state in fp32 and two 16-bit halves, so results are as accurate).
+
 Head dimensions above 256 (multiples of 256 up to 4096), 16-bit inputs, or float32 inputs with tf32 allowed:
 forward (float32 ``h``) and backward run on the tensor cores in two passes each (gated S x S matrices to scratch,
 then plain contractions: W V forward; dT K, dT^T Q, W^T dH backward).
