@@ -162,10 +162,19 @@ int round_inputs(const void** ptrs, int count, void* buf, int BH, int S, int D, 
 }
 
 // The CUDA-core arithmetic in two stages (simt_gemm.cu), where the caller's workspace has room for S x S matrices;
-// MLSTM_F_FORCE_SIMT and MLSTM_F_NO_SPLIT keep the one-stage kernel, which is the cross-check of everything else.
+// MLSTM_F_FORCE_SIMT and MLSTM_F_NO_SPLIT keep the one-stage kernel, which is the cross-check of everything else, and so do
+// head dimensions above 256, whose workspace without the tensor cores is promised to hold no S x S matrices.
 bool simt_two_stage(int S, int D, int dtype, int flags) {
     int rc;
-    return !(flags & (MLSTM_F_FORCE_SIMT | MLSTM_F_NO_SPLIT)) && pass_kind(S, D, dtype, flags, &rc) == KIND_SIMT && simt_gemm_supported(S);
+    return !(flags & (MLSTM_F_FORCE_SIMT | MLSTM_F_NO_SPLIT)) && D <= 256 &&
+           pass_kind(S, D, dtype, flags, &rc) == KIND_SIMT && simt_gemm_supported(S);
+}
+// Workspace queries answer for the arithmetic: where it is the CUDA cores' by itself, forcing them asks for no other size
+// (the one-stage kernel then leaves the matrices' part unused; the calls demand only what they use).
+int sizing_flags(int S, int D, int dtype, int flags) {
+    int rc;
+    const int unforced = flags & ~MLSTM_F_FORCE_SIMT;
+    return pass_kind(S, D, dtype, unforced, &rc) == KIND_SIMT && rc == MLSTM_OK ? unforced : flags;
 }
 // scratch of forward_impl behind the gate vectors: converted operands, or the two-stage form's matrices
 size_t fwd_extra_bytes(int BH, int S, int D, int dtype, int flags) {
@@ -301,7 +310,7 @@ size_t mlstm_mm_fwd_workspace(int B, int NH, int S, int D, int dtype, int flags)
     if (mm_fwd_two_pass(S, D, dtype, MLSTM_DT_F32, flags))
         return carve_fwd(nullptr, B * NH, S, false).bytes + two_pass_extra_bytes(B * NH, S, dtype);
     if (mm_chunk_route(B * NH, S, D, dtype, flags)) return mm_chunk_fwd_bytes(B * NH, S, D);
-    return carve_fwd(nullptr, B * NH, S, false).bytes + fwd_extra_bytes(B * NH, S, D, dtype, flags);
+    return carve_fwd(nullptr, B * NH, S, false).bytes + fwd_extra_bytes(B * NH, S, D, dtype, sizing_flags(S, D, dtype, flags));
 }
 
 int mlstm_mm_fwd(const void* q, const void* k, const void* v, const void* f, const void* i, void* h, float* m, float* b,
@@ -341,7 +350,7 @@ static size_t mm_bwd_workspace(int B, int NH, int S, int D, int dtype, int h_dty
     if (mm_chunk_route(B * NH, S, D, dtype, flags)) return mm_chunk_bwd_bytes(B * NH, S, D, dh_copy_bytes(dtype, h_dtype, gated) != 0);
     const size_t own = carve_bwd(nullptr, B * NH, S, D, dh_copy_bytes(dtype, h_dtype, gated)).bytes;
     if (mm_bwd_two_pass(S, D, dtype, flags)) return own + two_pass_bwd_extra_bytes(B * NH, S, D, dtype);
-    if (simt_two_stage(S, D, dtype, flags)) return own + simt_bwd_extra_bytes(B * NH, S, D);
+    if (simt_two_stage(S, D, dtype, sizing_flags(S, D, dtype, flags))) return own + simt_bwd_extra_bytes(B * NH, S, D);
     return own + tf32_copy_bytes(B * NH, S, D, dtype, flags, 4);
 }
 
