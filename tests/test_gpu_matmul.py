@@ -294,6 +294,38 @@ def test_autograd_function_with_output_gate(gc, dtype, D):
         gc.PKG.Triton_mLSTM.apply(t["q"], t["k"], t["v"], t["f"], t["i"], 32, 4, t["o"][..., :8])
 
 
+@pytest.mark.parametrize("which", ["dh", "o"])
+@pytest.mark.parametrize("entry,S,D,dtype", [
+    ("matmul", 130, 64, torch.float32), ("matmul", 256, 128, torch.bfloat16),
+    ("scan", 256, 128, torch.float16),       # the parallel kernels behind mlstm_scan
+    ("scan", 1280, 128, torch.bfloat16),     # the chunkwise backward
+])
+def test_gated_backward_takes_unaligned_gradients(gc, entry, S, D, dtype, which):
+    """A contiguous upstream gradient (or o) that starts one element behind a 16-byte boundary, as a view into a flat buffer
+    does: the same gradients as from an aligned one.  The gate's derivative then has a kernel of its own, with the same fp32
+    arithmetic up to the order of its products: a rounding of the gradients' type apart (bf16: 2^-8)."""
+    x = gc.make_inputs(1, 2, S, D, dtype, f_mean=2.0, qkv_scale=D ** -0.5, seed=S, with_o=True)
+    names = ("q", "k", "v", "f", "i", "o")
+
+    def run(off):
+        def place(t, shift):
+            buf = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")
+            view = buf[shift:shift + t.numel()].view(t.shape)
+            view.copy_(t)
+            assert view.is_contiguous() and (view.data_ptr() % 16 != 0) == (shift != 0)
+            return view
+        t = {n: place(x[n], off if n == which else 0).requires_grad_(True) for n in names}
+        if entry == "matmul":
+            h = gc.PKG.Triton_mLSTM.apply(*(t[n] for n in names[:5]), 32, 4, t["o"])
+        else:
+            h = gc.PKG.mlstm_scan(*(t[n] for n in names))
+        return torch.autograd.grad(h, [t[n] for n in names], place(x["dh"], off if which == "dh" else 0))
+
+    tol = 1e-5 if dtype == torch.float32 else 2.0 ** -8
+    for n, a, r in zip(names, run(1), run(0)):
+        assert orc.max_abs_rel(a.float(), r.float().cpu()) < tol, n
+
+
 @pytest.mark.parametrize("f_mean", [3.0, 0.0])
 def test_model_scale_slice_properties(gc, f_mean):
     """Configuration-4 shape per slice (S=4096, D=256, bf16) on a few slices, with retention-biased gates

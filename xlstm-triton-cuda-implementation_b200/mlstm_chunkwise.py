@@ -179,7 +179,7 @@ def mlstm_chunkwise_backward(dh, q, k, v, f, i, h, m, b, chunk_size=256):
 
 def _backward(dh, q, k, v, f, i, h, m, b, chunk_size, o=None):
     """(dq, dk, dv, df, di, do).  With the output gate ``o``, dh is the gradient of h * silu(o)."""
-    if o is not None and (o.data_ptr() & 15):    # the fused gate derivative reads 16 bytes at a time
+    if o is not None and ((o.data_ptr() | dh.data_ptr()) & 15):    # as in mlstm_matmul._backward
         from .mlstm_matmul import output_gate_backward
         dh, do = output_gate_backward(dh, h, o)
         return _backward(dh, q, k, v, f, i, h, m, b, chunk_size)[:5] + (do,)

@@ -92,7 +92,9 @@ def mlstm_matmul_backward(dh, q, k, v, f, i, h, m, b, flags=0):
 
 def _backward(dh, q, k, v, f, i, h, m, b, flags, o=None):
     """(dq, dk, dv, df, di, do).  With the output gate ``o``, dh is the gradient of h * silu(o)."""
-    if o is not None and (o.data_ptr() & 15):    # the fused gate derivative reads 16 bytes at a time
+    # the fused gate derivative reads 16 bytes at a time; the gate's own kernel takes any alignment (an upstream gradient may
+    # be a contiguous view into a flat buffer) and hands on an aligned dh
+    if o is not None and ((o.data_ptr() | dh.data_ptr()) & 15):
         dh, do = output_gate_backward(dh, h, o)
         return _backward(dh, q, k, v, f, i, h, m, b, flags)[:5] + (do,)
     dev = _lib.require_cuda(dh, q, k, v, f, i, h, m, b)
