@@ -253,6 +253,11 @@ int mlstm_read_status(const void* workspace, int* host_status, void* stream);
  * MLSTM_E_TIMEOUT, and the device stays usable.  `workspace`: at least 256 bytes. */
 int mlstm_selftest_wait_timeout(void* workspace, size_t workspace_bytes, long long limit_cycles, void* stream);
 
+/* Host-side check that guards the launch of the kernels that redistribute registers between their warps: MLSTM_OK when a
+ * kernel built with `registers_per_thread` registers can be launched, MLSTM_E_CUDA when its warps would wait for registers
+ * that the block does not have.  The launch makes the same check with the built kernel's own figure. */
+int mlstm_selftest_register_split(int registers_per_thread);
+
 #ifdef __cplusplus
 }
 #endif

@@ -63,6 +63,16 @@ def test_bad_arguments_rejected_without_a_device(pkg):
     assert b"aligned" in L.mlstm_status_string(-3)
 
 
+def test_register_split_is_refused_when_the_launch_cannot_cover_it(pkg):
+    """The chunkwise pair kernels raise their gate warps to 104 registers and lower the other four warps to 40: 58368 of the
+    block's 640 x 92 and more.  A build with fewer is refused before its launch."""
+    L = pkg._lib.lib()
+    split = 128 * 40 + 512 * 104
+    for regs in (40, 88, 91, 92, 96, 102):
+        assert (L.mlstm_selftest_register_split(regs) == 0) == (640 * regs >= split), regs
+    assert L.mlstm_selftest_register_split(88) == -6 and L.mlstm_selftest_register_split(96) == 0
+
+
 def test_python_wrappers_refuse_cpu_tensors(pkg):
     q = torch.zeros(1, 1, 8, 8)
     f = torch.zeros(1, 1, 8)

@@ -108,6 +108,8 @@ def lib():
     L.mlstm_ogate_fwd.argtypes = [vp, vp, vp, ctypes.c_longlong, i32, i32, vp]
     L.mlstm_ogate_bwd.restype = i32
     L.mlstm_ogate_bwd.argtypes = [vp] * 5 + [ctypes.c_longlong, i32, i32, vp]
+    L.mlstm_selftest_register_split.restype = i32
+    L.mlstm_selftest_register_split.argtypes = [i32]
     L.mlstm_selftest_wait_timeout.restype = i32
     L.mlstm_selftest_wait_timeout.argtypes = [vp, sz, ctypes.c_longlong, vp]
     L.mlstm_read_status.restype = i32
@@ -125,7 +127,8 @@ EXPORTS = [
     "mlstm_chunk_workspace", "mlstm_chunk_gate_summary", "mlstm_chunk_prepare", "mlstm_chunk_local_state",
     "mlstm_chunk_apply", "mlstm_chunk_sp_record_floats", "mlstm_chunk_sp_local", "mlstm_chunk_sp_apply",
     "mlstm_chunk_read_mb", "mlstm_chunk_bwd_workspace", "mlstm_chunk_bwd",
-    "mlstm_step_max_tokens", "mlstm_step", "mlstm_forward_f16_static_status", "mlstm_selftest_wait_timeout", "mlstm_ogate_fwd", "mlstm_ogate_bwd",
+    "mlstm_step_max_tokens", "mlstm_step", "mlstm_forward_f16_static_status", "mlstm_selftest_wait_timeout", "mlstm_selftest_register_split",
+    "mlstm_ogate_fwd", "mlstm_ogate_bwd",
 ]
 
 

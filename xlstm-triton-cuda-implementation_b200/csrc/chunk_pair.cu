@@ -40,7 +40,12 @@ constexpr int NTHREADS = 128 + NGATE;           // a warpgroup with the producer
 // values come back through L2, the shared memory leaves L1 nothing to speak of: 300 cycles each), so the first
 // warpgroup gives most of its share away: 128 x 40 + 512 x 104 of the 640 x 96 the block is launched with.
 constexpr int REGS_ROLE = 40, REGS_GATE = 104;
-static_assert(128 * REGS_ROLE + NGATE * REGS_GATE <= NTHREADS * 96, "setmaxnreg draws on the registers of the launch");
+// An increase that the block was not launched with waits for ever, in front of every bounded wait: what the built kernel
+// really has is checked on the host before its first launch.
+constexpr bool register_split_fits(int regs_at_launch) {
+    return REGS_ROLE <= regs_at_launch && 128 * REGS_ROLE + NGATE * REGS_GATE <= NTHREADS * regs_at_launch;
+}
+static_assert(register_split_fits(96), "setmaxnreg draws on the registers of the launch");
 constexpr int BOX_BYTES = 128 * 128;           // 128 rows x 128 bytes
 constexpr int HBOX_BYTES = 64 * 128;           // 64 rows x 128 bytes (half of a streamed Y tile's rows)
 constexpr long long WAIT_LIMIT = 4000000000LL;
@@ -832,7 +837,14 @@ int launch_chunk_pair_one(const PassParams& p, int in_dtype, cudaStream_t st) {
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MLSTM_E_CUDA;
         if (!opted[dev].load(std::memory_order_acquire)) {
-            cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+            cudaFuncAttributes fa;
+            cudaError_t ce = cudaFuncGetAttributes(&fa, kern);
+            if (ce == cudaSuccess && !register_split_fits(fa.numRegs)) ce = cudaErrorLaunchOutOfResources;
+            if (ce != cudaSuccess) {
+                cudaGetLastError();
+                return note_cuda_error(ce, "registers of mlstm_chunk_pair at launch against its register split");
+            }
+            ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
             if (ce != cudaSuccess) {
                 cudaGetLastError();
                 return note_cuda_error(ce, "cudaFuncSetAttribute(MaxDynamicSharedMemorySize)");
@@ -891,3 +903,7 @@ int launch_chunk_pair(int mode, const PassParams& p, int in_dtype, int out_dtype
 }
 
 }  // namespace mlstm
+
+extern "C" int mlstm_selftest_register_split(int registers_per_thread) {
+    return mlstm::register_split_fits(registers_per_thread) ? MLSTM_OK : MLSTM_E_CUDA;
+}
