@@ -52,6 +52,39 @@ def test_workspace_sizes_and_support_matrix(pkg):
     assert L.mlstm_tc_supported(4096, 96, 2) == 0
 
 
+def test_chunkwise_route_bounds_its_states(pkg):
+    """Long bf16 sequences behind the parallel entry points: block states of at most 512 MB per set (one set forward, two
+    backward) beside the row vectors that the quadratic kernels need as well, whatever the number of slices."""
+    L, FORCE_TC, MB = pkg._lib.lib(), pkg._lib.F_FORCE_TC, 1 << 20
+    for B, NH, S, D in ((16, 8, 4096, 256), (32, 8, 131072, 256), (255, 16, 8192, 256), (64, 8, 65536, 128)):
+        slack = 8 * MB + B * NH * S             # vector states, block boundaries, segments of the gate scan
+        fwd = L.mlstm_mm_fwd_workspace(B, NH, S, D, 2, 0) - L.mlstm_mm_fwd_workspace(B, NH, S, D, 2, FORCE_TC)
+        assert 0 < fwd <= 512 * MB + slack, (B, NH, S, D, fwd)
+        for query in (L.mlstm_mm_bwd_workspace, L.mlstm_mm_bwd_ogate_workspace):
+            bwd = query(B, NH, S, D, 2, 0, 0) - query(B, NH, S, D, 2, 0, FORCE_TC)
+            assert 0 < bwd <= 1024 * MB + slack, (B, NH, S, D, bwd)
+
+
+def test_workspace_falls_back_to_the_quadratic_form(pkg, monkeypatch):
+    """Where the chunkwise form's states do not fit the memory the call asks for the quadratic kernels; nothing else does."""
+    lib, L = pkg._lib, pkg._lib.lib()
+    query = lambda fl: L.mlstm_mm_fwd_workspace(1, 1, 8 << 20, 256, 2, fl)     # one slice: 8 GB of states
+    room = 1 << 30
+
+    def alloc(nbytes, dev):
+        if nbytes > room:
+            raise torch.OutOfMemoryError("no room")
+        return nbytes
+    monkeypatch.setattr(lib, "workspace", alloc)
+    assert lib.workspace_for(query, 0, "cuda") == (query(lib.F_FORCE_TC), lib.F_FORCE_TC)
+    room = 1 << 40
+    assert lib.workspace_for(query, 0, "cuda") == (query(0), 0)
+    room = 1 << 20
+    for q in (query, lambda fl: L.mlstm_mm_fwd_workspace(1, 8, 4096, 32, 0, fl)):   # (fp32, D = 32: no quadratic tensor-core form)
+        with pytest.raises(torch.OutOfMemoryError):
+            lib.workspace_for(q, 0, "cuda")
+
+
 def test_bad_arguments_rejected_without_a_device(pkg):
     L = pkg._lib.lib()
     one = ctypes.c_void_p(16)  # non-null, aligned; never dereferenced because checks fail first

@@ -422,6 +422,26 @@ def test_long_sequences_take_the_chunkwise_form(gc, BH, S, D, gated, pad):
             assert err(cut(a), r) < 1.25 * err(cut(a2), r), name
 
 
+def test_chunkwise_route_in_slice_groups(gc):
+    """More states than a set may hold (512 MB): the slices go in two groups of 33.  A slice's results do not depend on the
+    slices beside it: both groups equal the same slices called on their own, in one group each."""
+    BH, S, D, cut = 66, 8100, 256, 33
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda *shape: torch.randn(shape, device="cuda", generator=g)
+    q, k, v, o = ((rnd(1, BH, S, D) * s).bfloat16() for s in (D ** -0.5, D ** -0.5, D ** -0.5, 1.0))
+    f, i, dh = (3.0 + rnd(1, BH, S)).bfloat16(), rnd(1, BH, S).bfloat16(), rnd(1, BH, S, D)
+    backward = gc.PKG.mlstm_matmul.__globals__["_backward"]
+
+    def run(sl):
+        x = [t[:, sl].contiguous() for t in (q, k, v, f, i)]
+        h, m, b = gc.PKG.mlstm_matmul_forward(*x)
+        return (h, m, b) + backward(dh[:, sl].contiguous(), *x, h, m, b, 0, o[:, sl].contiguous())
+    whole = run(slice(0, BH))
+    for sl in (slice(0, cut), slice(cut, BH)):
+        for a, part in zip(whole, run(sl)):
+            assert torch.equal(a[:, sl], part)
+
+
 @pytest.mark.parametrize("B,NH,S,D,dtype", [
     (1, 2, 64, 8, torch.float32),          # one tile
     (2, 1, 65, 32, torch.float32),         # a tile and one row

@@ -175,6 +175,20 @@ def workspace(nbytes: int, dev) -> torch.Tensor:
     return buf
 
 
+def workspace_for(query, flags: int, dev):
+    """(workspace, flags) of a call whose scratch size is ``query(flags)``.  Where the memory does not hold the scratch of the
+    form the library would choose (the chunkwise form of long sequences keeps block states) but does hold that of the
+    quadratic tensor-core kernels, the flags returned ask for those."""
+    nbytes = query(flags)
+    try:
+        return workspace(nbytes, dev), flags
+    except torch.OutOfMemoryError:
+        less = query(flags | F_FORCE_TC)
+        if not 0 < less < nbytes:
+            raise
+    return workspace(less, dev), flags | F_FORCE_TC
+
+
 def check(code: int, where: str):
     if code != 0:
         raise MlstmError(code, where)

@@ -227,8 +227,8 @@ struct ChunkWs {
 };
 
 // parts: 16-bit matrices a carried state is held in.  2: written by launch_carried_states, and what only the stages of
-// the 1-part form use is left out
-ChunkWs carve(void* ws, int BH, int S, int D, int chunk, int parts = 1) {
+// the 1-part form use is left out; states of `group` slices at a time (0: all), m and b are the caller's
+ChunkWs carve(void* ws, int BH, int S, int D, int chunk, int parts = 1, int group = 0) {
     ChunkWs w{};
     uint8_t* base = static_cast<uint8_t*>(ws);
     size_t off = 0;
@@ -240,15 +240,17 @@ ChunkWs carve(void* ws, int BH, int S, int D, int chunk, int parts = 1) {
     const size_t Spad = round_up(S, TILE);
     const size_t vec = static_cast<size_t>(BH) * Spad * sizeof(float);
     w.NB = (S + chunk - 1) / chunk;
-    const size_t nblk = static_cast<size_t>(BH) * w.NB;
+    const size_t nblk = static_cast<size_t>(group ? group : BH) * w.NB;
     w.status = static_cast<int*>(take(WS_ALIGN));
     w.ga = static_cast<float*>(take(vec));
     w.gAn = static_cast<float*>(take(vec));
     w.gaw = static_cast<float*>(take(vec));
     w.a_ref = static_cast<double*>(take(vec / REF_BLOCK * 2));
     w.An_ref = static_cast<double*>(take(vec / REF_BLOCK * 2));
-    w.m = static_cast<float*>(take(static_cast<size_t>(BH) * S * sizeof(float)));
-    w.b = static_cast<float*>(take(static_cast<size_t>(BH) * S * sizeof(float)));
+    if (parts == 1) {
+        w.m = static_cast<float*>(take(static_cast<size_t>(BH) * S * sizeof(float)));
+        w.b = static_cast<float*>(take(static_cast<size_t>(BH) * S * sizeof(float)));
+    }
     w.An_bound = static_cast<double*>(take(static_cast<size_t>(BH) * (w.NB + 1) * sizeof(double)));
     const size_t gs = gates_scratch_bytes(BH, static_cast<int>(Spad));
     w.gscratch = gs ? static_cast<double*>(take(gs)) : nullptr;
@@ -267,6 +269,17 @@ ChunkWs carve(void* ws, int BH, int S, int D, int chunk, int parts = 1) {
         w.z_in = static_cast<float*>(take(static_cast<size_t>(BH) * D * sizeof(float)));
     }
     w.bytes = off;
+    return w;
+}
+
+// the same workspace as the slices from bh0 on see it; the states are those of whatever group is being worked on
+ChunkWs from_slice(ChunkWs w, int bh0, int S) {
+    const size_t Spad = round_up(S, TILE), vec = bh0 * Spad, ref = bh0 * (Spad / REF_BLOCK), row = static_cast<size_t>(bh0) * S;
+    w.ga += vec; w.gAn += vec; w.gaw += vec;
+    w.a_ref += ref; w.An_ref += ref;
+    w.An_bound += static_cast<size_t>(bh0) * (w.NB + 1);
+    if (w.m) w.m += row;
+    if (w.b) w.b += row;
     return w;
 }
 
@@ -442,9 +455,9 @@ struct ChunkBwdWs {
     void *rstatesT;    // 1 part: transposed copy of the states carried back
     size_t bytes;
 };
-static ChunkBwdWs carve_bwd_chunk(void* ws, int BH, int S, int D, int chunk, bool need_dh16, int parts = 1) {
+static ChunkBwdWs carve_bwd_chunk(void* ws, int BH, int S, int D, int chunk, bool need_dh16, int parts = 1, int group = 0) {
     ChunkBwdWs w{};
-    w.f = carve(ws, BH, S, D, chunk, parts);
+    w.f = carve(ws, BH, S, D, chunk, parts, group);
     uint8_t* base = static_cast<uint8_t*>(ws);
     size_t off = w.f.bytes;
     auto take = [&](size_t bytes) {
@@ -453,7 +466,7 @@ static ChunkBwdWs carve_bwd_chunk(void* ws, int BH, int S, int D, int chunk, boo
         return p;
     };
     const size_t vec = static_cast<size_t>(BH) * round_up(S, TILE) * sizeof(float);
-    const size_t nblk = static_cast<size_t>(BH) * w.f.NB;
+    const size_t nblk = static_cast<size_t>(group ? group : BH) * w.f.NB;
     w.gB = static_cast<float*>(take(vec));
     w.gBw = static_cast<float*>(take(vec));
     w.g = static_cast<float*>(take(vec));
@@ -477,75 +490,84 @@ size_t mlstm_chunk_bwd_ogate_workspace(int B, int NH, int S, int D, int dtype, i
     return carve_bwd_chunk(nullptr, B * NH, S, D, chunk, true).bytes;
 }
 
-// (arguments checked, workspace carved by the caller)
+// (arguments checked, workspace carved by the caller with the same `parts` and `group`)
 static int chunk_bwd_core(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h,
                           const float* m, const float* b, const void* o, void* d_o, void* dq, void* dk, void* dv, void* df, void* di,
-                          const ChunkBwdWs& w, int BH, int S, int D, int dtype, int h_dtype, int chunk, int parts, cudaStream_t st) {
+                          const ChunkBwdWs& w, int BH, int S, int D, int dtype, int h_dtype, int chunk, int parts, int group,
+                          cudaStream_t st) {
     const int Spad = round_up(S, TILE);
-    const ChunkWs& c = w.f;
     int rc;
-    // gates and forward states, as in the forward (the gate pass also clears the status word and the work-item counters)
-    if ((rc = launch_gates_fwd(f, i, c.ga, c.gAn, c.a_ref, c.An_ref, nullptr, BH, S, Spad, dtype, st, nullptr, nullptr,
-                               c.An_bound, chunk, c.gscratch, c.gaw, c.status, STATUS_WORDS)) != MLSTM_OK)
+    // gates, as in the forward (the gate pass also clears the status word and the work-item counters)
+    if ((rc = launch_gates_fwd(f, i, w.f.ga, w.f.gAn, w.f.a_ref, w.f.An_ref, nullptr, BH, S, Spad, dtype, st, nullptr, nullptr,
+                               w.f.An_bound, chunk, w.f.gscratch, w.f.gaw, w.f.status, STATUS_WORDS)) != MLSTM_OK)
+        return rc;
+    // delta = dh . h, n, db -> the backward's per-row vectors (and dh in the input type)
+    if ((rc = launch_bwd_prep(h, dh, b, m, w.f.gAn, w.gB, w.gBw, w.g, w.dh16, o, d_o, BH, S, Spad, D, h_dtype, dtype, st)) != MLSTM_OK)
         return rc;
     // Two parts: every pass on CTA pairs, which read the states as they are.  One part: dQ and dK on the one-CTA kernel (its
     // state step contracts over transposed states).  df is a running sum of differences of the row dots of these two passes,
     // in which the rounding of a 16-bit state's path adds up (1 to 4 % of df at S = 16384, whatever the order): this entry
     // keeps the rounding it has always had there, and with it its results.
     const bool two = parts == 2;
-    BlockStateArgs fwd = forward_states(k, v, c, BH, S, Spad, chunk);
-    if (two) {
-        fwd.U = w.fstates; fwd.vec = c.zstate;
-        if ((rc = launch_carried_states(fwd, D, dtype, st)) != MLSTM_OK) return rc;
-    } else {
-        if ((rc = launch_identity(c.ident, D, dtype, st)) != MLSTM_OK) return rc;
-        if ((rc = launch_block_states(fwd, D, dtype, st)) != MLSTM_OK) return rc;
-        if ((rc = launch_state_scan(c.U, c.zU, c.An_bound, nullptr, nullptr, nullptr, c.zstate, nullptr, nullptr, BH, c.NB, D, dtype, st,
-                                    nullptr, nullptr, 0, nullptr, w.fstates, 0)) != MLSTM_OK)
-            return rc;
+    if (!two && (rc = launch_identity(w.f.ident, D, dtype, st)) != MLSTM_OK) return rc;
+    for (int bh0 = 0; bh0 < BH; bh0 += group) {
+        const int n = BH - bh0 < group ? BH - bh0 : group;
+        const ChunkWs c = from_slice(w.f, bh0, S);
+        const size_t vec = static_cast<size_t>(bh0) * Spad, at16 = static_cast<size_t>(bh0) * S * D * 2;   // (dh in 16 bits here)
+        auto in = [&](const void* x) { return static_cast<const void*>(static_cast<const uint8_t*>(x) + at16); };
+        auto out = [&](void* x) { return static_cast<void*>(static_cast<uint8_t*>(x) + at16); };
+        const void *qs = in(q), *ks = in(k), *vs = in(v), *dhs = in(w.dh16 ? w.dh16 : dh);
+        const float *gB = w.gB + vec, *gBw = w.gBw + vec, *g = w.g + vec;
+        // forward states, as in the forward
+        BlockStateArgs fwd = forward_states(ks, vs, c, n, S, Spad, chunk);
+        if (two) {
+            fwd.U = w.fstates; fwd.vec = c.zstate;
+            if ((rc = launch_carried_states(fwd, D, dtype, st)) != MLSTM_OK) return rc;
+        } else {
+            if ((rc = launch_block_states(fwd, D, dtype, st)) != MLSTM_OK) return rc;
+            if ((rc = launch_state_scan(c.U, c.zU, c.An_bound, nullptr, nullptr, nullptr, c.zstate, nullptr, nullptr, n, c.NB, D, dtype, st,
+                                        nullptr, nullptr, 0, nullptr, w.fstates, 0)) != MLSTM_OK)
+                return rc;
+        }
+        // the state carried back, R_k [key, value] and r_k: the recurrence in reverse over what every block contributes,
+        // P_k = sum_t beta_t q_t dh_t^T, p_k = sum_t beta_t g_t q_t with beta_t = exp(A_end(k-1) - A_t) scale / n_t, g_t = db_t n_t
+        BlockStateArgs bwd = fwd;
+        bwd.X = qs; bwd.Y = dhs; bwd.col_w = gBw; bwd.col_ref = c.An_ref; bwd.col_g = g; bwd.reverse = 1;
+        if (two) {
+            bwd.U = c.states; bwd.vec = w.rvec;
+            if ((rc = launch_carried_states(bwd, D, dtype, st)) != MLSTM_OK) return rc;
+        } else {
+            if ((rc = launch_block_states(bwd, D, dtype, st)) != MLSTM_OK) return rc;
+            if ((rc = launch_state_scan(c.U, c.zU, c.An_bound, nullptr, nullptr, c.states, w.rvec, nullptr, nullptr, n, c.NB, D, dtype, st,
+                                        nullptr, nullptr, 0, nullptr, w.rstatesT, 1)) != MLSTM_OK)
+                return rc;
+        }
+        PassParams p{};
+        p.S = S; p.Spad = Spad; p.BH = n; p.D = D; p.status = c.status; p.sched = c.status + 8; p.sched_zeroed = 1;
+        p.chunk_tiles = chunk / TILE; p.NB = c.NB; p.An_bound = c.An_bound; p.ident = c.ident; p.state_parts = parts;
+        p.dot_part_stride = static_cast<long long>(BH) * Spad;
+        auto pass = [&](int mode, bool pair) {
+            return pair ? launch_chunk_pair(mode, p, dtype, dtype, st) : launch_pass_tc(mode, p, dtype, dtype, st);
+        };
+        // dQ = ((dH V^T + g_r) * decay) K within the block, + beta (S_k dh + g z_k) from the inbound state
+        p.X = dhs; p.Y = vs; p.Z = ks;
+        p.row_rel = gB; p.row_ref = c.An_ref; p.row_g = g; p.col_rel = c.ga; p.col_w = c.gaw; p.col_ref = c.a_ref; p.col_g = nullptr;
+        p.states = w.fstates; p.zstate = c.zstate;
+        p.out = out(dq); p.dot_src = qs; p.dot_out = w.Rdot + vec;
+        if ((rc = pass(DQC, two)) != MLSTM_OK) return rc;
+        // dK = ((V dH^T + g_c) * decay) Q within the block, + gamma (R_k v + r_k) from the later blocks
+        p.X = vs; p.Y = dhs; p.Z = qs;
+        p.row_rel = c.ga; p.row_ref = c.a_ref; p.row_g = nullptr; p.col_rel = gB; p.col_w = gBw; p.col_ref = c.An_ref; p.col_g = g;
+        p.states = two ? c.states : w.rstatesT; p.rvec = w.rvec;
+        p.out = out(dk); p.dot_src = ks; p.dot_out = w.dI + vec;
+        if ((rc = pass(DKC, two)) != MLSTM_OK) return rc;
+        // dV = ((K Q^T) * decay / n) dH within the block, + gamma R_k^T k from the later blocks
+        p.X = ks; p.Y = qs; p.Z = dhs;
+        p.col_g = nullptr; p.states = c.states;
+        p.out = out(dv); p.dot_src = nullptr; p.dot_out = nullptr;
+        if ((rc = pass(DVC, chunk_pair_supported(D, dtype, p.chunk_tiles))) != MLSTM_OK) return rc;
     }
-    // delta = dh . h, n, db -> the backward's per-row vectors (and dh in the input type)
-    if ((rc = launch_bwd_prep(h, dh, b, m, c.gAn, w.gB, w.gBw, w.g, w.dh16, o, d_o, BH, S, Spad, D, h_dtype, dtype, st)) != MLSTM_OK)
-        return rc;
-    const void* dhp = w.dh16 ? w.dh16 : dh;
-    // the state carried back, R_k [key, value] and r_k: the recurrence in reverse over what every block contributes,
-    // P_k = sum_t beta_t q_t dh_t^T, p_k = sum_t beta_t g_t q_t with beta_t = exp(A_end(k-1) - A_t) scale / n_t, g_t = db_t n_t
-    BlockStateArgs bwd = fwd;
-    bwd.X = q; bwd.Y = dhp; bwd.col_w = w.gBw; bwd.col_ref = c.An_ref; bwd.col_g = w.g; bwd.reverse = 1;
-    if (two) {
-        bwd.U = c.states; bwd.vec = w.rvec;
-        if ((rc = launch_carried_states(bwd, D, dtype, st)) != MLSTM_OK) return rc;
-    } else {
-        if ((rc = launch_block_states(bwd, D, dtype, st)) != MLSTM_OK) return rc;
-        if ((rc = launch_state_scan(c.U, c.zU, c.An_bound, nullptr, nullptr, c.states, w.rvec, nullptr, nullptr, BH, c.NB, D, dtype, st,
-                                    nullptr, nullptr, 0, nullptr, w.rstatesT, 1)) != MLSTM_OK)
-            return rc;
-    }
-    PassParams p{};
-    p.S = S; p.Spad = Spad; p.BH = BH; p.D = D; p.status = c.status; p.sched = c.status + 8; p.sched_zeroed = 1;
-    p.chunk_tiles = chunk / TILE; p.NB = c.NB; p.An_bound = c.An_bound; p.ident = c.ident; p.state_parts = parts;
-    p.dot_part_stride = static_cast<long long>(BH) * Spad;
-    // dQ = ((dH V^T + g_r) * decay) K within the block, + beta (S_k dh + g z_k) from the inbound state
-    auto pass = [&](int mode, bool pair) {
-        return pair ? launch_chunk_pair(mode, p, dtype, dtype, st) : launch_pass_tc(mode, p, dtype, dtype, st);
-    };
-    p.X = dhp; p.Y = v; p.Z = k;
-    p.row_rel = w.gB; p.row_ref = c.An_ref; p.row_g = w.g; p.col_rel = c.ga; p.col_w = c.gaw; p.col_ref = c.a_ref; p.col_g = nullptr;
-    p.states = w.fstates; p.zstate = c.zstate;
-    p.out = dq; p.dot_src = q; p.dot_out = w.Rdot;
-    if ((rc = pass(DQC, two)) != MLSTM_OK) return rc;
-    // dK = ((V dH^T + g_c) * decay) Q within the block, + gamma (R_k v + r_k) from the later blocks
-    p.X = v; p.Y = dhp; p.Z = q;
-    p.row_rel = c.ga; p.row_ref = c.a_ref; p.row_g = nullptr; p.col_rel = w.gB; p.col_w = w.gBw; p.col_ref = c.An_ref; p.col_g = w.g;
-    p.states = two ? c.states : w.rstatesT; p.rvec = w.rvec;
-    p.out = dk; p.dot_src = k; p.dot_out = w.dI;
-    if ((rc = pass(DKC, two)) != MLSTM_OK) return rc;
-    // dV = ((K Q^T) * decay / n) dH within the block, + gamma R_k^T k from the later blocks
-    p.X = k; p.Y = q; p.Z = dhp;
-    p.col_g = nullptr; p.states = c.states;
-    p.out = dv; p.dot_src = nullptr; p.dot_out = nullptr;
-    if ((rc = pass(DVC, chunk_pair_supported(D, dtype, p.chunk_tiles))) != MLSTM_OK) return rc;
-    return launch_df(f, w.dI, w.Rdot, df, di, BH, S, Spad, dtype, st, TC_DOT_PARTS, static_cast<long long>(BH) * Spad, c.gscratch);
+    return launch_df(f, w.dI, w.Rdot, df, di, BH, S, Spad, dtype, st, TC_DOT_PARTS, static_cast<long long>(BH) * Spad, w.f.gscratch);
 }
 
 static int chunk_bwd_impl(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h,
@@ -562,7 +584,7 @@ static int chunk_bwd_impl(const void* dh, const void* q, const void* k, const vo
     // dh in the input type, taken through the output gate where there is one
     ChunkBwdWs w = carve_bwd_chunk(workspace, B * NH, S, D, chunk, o || h_dtype != dtype);
     if (!workspace || workspace_bytes < w.bytes || !aligned16(workspace)) return MLSTM_E_WORKSPACE;
-    return chunk_bwd_core(dh, q, k, v, f, i, h, m, b, o, d_o, dq, dk, dv, df, di, w, B * NH, S, D, dtype, h_dtype, chunk, 1,
+    return chunk_bwd_core(dh, q, k, v, f, i, h, m, b, o, d_o, dq, dk, dv, df, di, w, B * NH, S, D, dtype, h_dtype, chunk, 1, B * NH,
                           static_cast<cudaStream_t>(stream));
 }
 
@@ -666,11 +688,26 @@ bool mm_chunk_route(int BH, int S, int D, int dtype, int flags) {
     return S >= 2048 && static_cast<long long>(BH) * S >= 131072;
 }
 
-size_t mm_chunk_fwd_bytes(int BH, int S, int D) { return carve(nullptr, BH, S, D, MM_CHUNK, 2).bytes; }
+// Slices whose states are in the workspace at one time.  A state costs 4 D bytes per position of its slice (two 16-bit
+// matrices per block of 256), so slices go in groups of at most MM_STATE_BYTES of one set of states, of about the same size;
+// a slice that is longer than that goes alone.  One set forward, two backward (S_k and R_k).  At B = 16, NH = 8, S = 4096,
+// D = 256 a set is just one group.
+constexpr size_t MM_STATE_BYTES = size_t{512} << 20;
+static int mm_chunk_group(int BH, int S, int D) {
+    const size_t one = static_cast<size_t>((S + MM_CHUNK - 1) / MM_CHUNK) * D * D * 2 * 2;
+    const size_t most = one < MM_STATE_BYTES ? MM_STATE_BYTES / one : 1;
+    const int groups = static_cast<int>((BH + most - 1) / most);
+    return (BH + groups - 1) / groups;
+}
+
+size_t mm_chunk_fwd_bytes(int BH, int S, int D) {
+    return carve(nullptr, BH, S, D, MM_CHUNK, 2, mm_chunk_group(BH, S, D)).bytes;
+}
 
 int mm_chunk_fwd(const void* q, const void* k, const void* v, const void* f, const void* i, void* h, float* m, float* b, void* workspace,
                  int BH, int S, int D, int dtype, int h_dtype, cudaStream_t st) {
-    ChunkWs w = carve(workspace, BH, S, D, MM_CHUNK, 2);
+    const int group = mm_chunk_group(BH, S, D);
+    ChunkWs w = carve(workspace, BH, S, D, MM_CHUNK, 2, group);
     w.m = m;
     w.b = b;
     const int Spad = round_up(S, TILE);
@@ -679,21 +716,31 @@ int mm_chunk_fwd(const void* q, const void* k, const void* v, const void* f, con
     if ((rc = launch_gates_fwd(f, i, w.ga, w.gAn, w.a_ref, w.An_ref, m, BH, S, Spad, dtype, st, nullptr, nullptr, w.An_bound, MM_CHUNK,
                                w.gscratch, w.gaw, w.status, STATUS_WORDS)) != MLSTM_OK)
         return rc;
-    BlockStateArgs a = forward_states(k, v, w, BH, S, Spad, MM_CHUNK);
-    a.U = w.states; a.vec = w.zstate;
-    if ((rc = launch_carried_states(a, D, dtype, st)) != MLSTM_OK) return rc;
-    return launch_fwdc(q, k, v, nullptr, h, h_dtype, w, BH, S, Spad, D, dtype, MM_CHUNK, nullptr, st, 2);
+    for (int bh0 = 0; bh0 < BH; bh0 += group) {
+        const int n = BH - bh0 < group ? BH - bh0 : group;
+        const size_t at = static_cast<size_t>(bh0) * S * D;
+        auto in = [&](const void* x) { return static_cast<const void*>(static_cast<const uint8_t*>(x) + at * 2); };
+        const ChunkWs c = from_slice(w, bh0, S);
+        BlockStateArgs a = forward_states(in(k), in(v), c, n, S, Spad, MM_CHUNK);
+        a.U = c.states; a.vec = c.zstate;
+        if ((rc = launch_carried_states(a, D, dtype, st)) != MLSTM_OK) return rc;
+        void* hs = static_cast<uint8_t*>(h) + at * (h_dtype == MLSTM_DT_F32 ? 4 : 2);
+        if ((rc = launch_fwdc(in(q), in(k), in(v), nullptr, hs, h_dtype, c, n, S, Spad, D, dtype, MM_CHUNK, nullptr, st, 2)) != MLSTM_OK)
+            return rc;
+    }
+    return MLSTM_OK;
 }
 
 size_t mm_chunk_bwd_bytes(int BH, int S, int D, bool dh_copy) {
-    return carve_bwd_chunk(nullptr, BH, S, D, MM_CHUNK, dh_copy, 2).bytes;
+    return carve_bwd_chunk(nullptr, BH, S, D, MM_CHUNK, dh_copy, 2, mm_chunk_group(BH, S, D)).bytes;
 }
 
 int mm_chunk_bwd(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i, const void* h, const float* m,
                  const float* b, const void* o, void* d_o, void* dq, void* dk, void* dv, void* df, void* di, void* workspace, int BH,
                  int S, int D, int dtype, int h_dtype, cudaStream_t st) {
-    const ChunkBwdWs w = carve_bwd_chunk(workspace, BH, S, D, MM_CHUNK, o || h_dtype != dtype, 2);
-    return chunk_bwd_core(dh, q, k, v, f, i, h, m, b, o, d_o, dq, dk, dv, df, di, w, BH, S, D, dtype, h_dtype, MM_CHUNK, 2, st);
+    const int group = mm_chunk_group(BH, S, D);
+    const ChunkBwdWs w = carve_bwd_chunk(workspace, BH, S, D, MM_CHUNK, o || h_dtype != dtype, 2, group);
+    return chunk_bwd_core(dh, q, k, v, f, i, h, m, b, o, d_o, dq, dk, dv, df, di, w, BH, S, D, dtype, h_dtype, MM_CHUNK, 2, group, st);
 }
 
 }  // namespace mlstm

@@ -75,7 +75,7 @@ def mlstm_matmul_forward(q, k, v, f, i, h_dtype=torch.float32, flags=0):
     m = torch.empty((B, NH, S), device=dev, dtype=torch.float32)
     b = torch.empty((B, NH, S), device=dev, dtype=torch.float32)
     L = _lib.lib()
-    ws = _lib.workspace(L.mlstm_mm_fwd_workspace(B, NH, S, D, dt, flags), dev)
+    ws, flags = _lib.workspace_for(lambda fl: L.mlstm_mm_fwd_workspace(B, NH, S, D, dt, fl), flags, dev)
     with torch.cuda.device(dev):
         rc = L.mlstm_mm_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), f.data_ptr(), i.data_ptr(), h.data_ptr(),
                             m.data_ptr(), b.data_ptr(), ws.data_ptr(), ws.numel(), B, NH, S, D, dt,
@@ -105,13 +105,12 @@ def _backward(dh, q, k, v, f, i, h, m, b, flags, o=None):
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
     df, di = torch.empty_like(f), torch.empty_like(i)
     L = _lib.lib()
-    if o is None:
-        do = None
-        ws = _lib.workspace(L.mlstm_mm_bwd_workspace(B, NH, S, D, dt, hdt, flags), dev)
-    else:
+    do = None
+    if o is not None:
         _lib.require_cuda(q, o)
         do = torch.empty_like(o)
-        ws = _lib.workspace(L.mlstm_mm_bwd_ogate_workspace(B, NH, S, D, dt, hdt, flags), dev)
+    query = L.mlstm_mm_bwd_workspace if o is None else L.mlstm_mm_bwd_ogate_workspace
+    ws, flags = _lib.workspace_for(lambda fl: query(B, NH, S, D, dt, hdt, fl), flags, dev)
     with torch.cuda.device(dev):
         if o is not None:
             rc = L.mlstm_mm_bwd_ogate(dh.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), f.data_ptr(), i.data_ptr(),
