@@ -501,9 +501,6 @@ static int chunk_bwd_core(const void* dh, const void* q, const void* k, const vo
     if ((rc = launch_gates_fwd(f, i, w.f.ga, w.f.gAn, w.f.a_ref, w.f.An_ref, nullptr, BH, S, Spad, dtype, st, nullptr, nullptr,
                                w.f.An_bound, chunk, w.f.gscratch, w.f.gaw, w.f.status, STATUS_WORDS)) != MLSTM_OK)
         return rc;
-    // delta = dh . h, n, db -> the backward's per-row vectors (and dh in the input type)
-    if ((rc = launch_bwd_prep(h, dh, b, m, w.f.gAn, w.gB, w.gBw, w.g, w.dh16, o, d_o, BH, S, Spad, D, h_dtype, dtype, st)) != MLSTM_OK)
-        return rc;
     // Two parts: every pass on CTA pairs, which read the states as they are.  One part: dQ and dK on the one-CTA kernel (its
     // state step contracts over transposed states).  df is a running sum of differences of the row dots of these two passes,
     // in which the rounding of a 16-bit state's path adds up (1 to 4 % of df at S = 16384, whatever the order): this entry
@@ -529,6 +526,11 @@ static int chunk_bwd_core(const void* dh, const void* q, const void* k, const vo
                                         nullptr, nullptr, 0, nullptr, w.fstates, 0)) != MLSTM_OK)
                 return rc;
         }
+        // delta = dh . h, n, db -> the backward's per-row vectors of all slices (and dh in the input type).  Here, right in front
+        // of the pass that reads them: in front of the forward states it cost 5 of 466 us at NH = 8, S = 16384, D = 128
+        if (bh0 == 0 && (rc = launch_bwd_prep(h, dh, b, m, w.f.gAn, w.gB, w.gBw, w.g, w.dh16, o, d_o, BH, S, Spad, D, h_dtype, dtype,
+                                              st)) != MLSTM_OK)
+            return rc;
         // the state carried back, R_k [key, value] and r_k: the recurrence in reverse over what every block contributes,
         // P_k = sum_t beta_t q_t dh_t^T, p_k = sum_t beta_t g_t q_t with beta_t = exp(A_end(k-1) - A_t) scale / n_t, g_t = db_t n_t
         BlockStateArgs bwd = fwd;
