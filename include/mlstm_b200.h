@@ -11,6 +11,9 @@
  * device state of its own, with one exception: mlstm_forward_f16_static() works in a fixed array
  * inside the library's device image (see there).  Host-side caches (tensor-map encoder entry point,
  * per-device kernel attributes) are guarded for concurrent callers.
+ * Input gates may be -inf (left padding): such a position contributes nothing, and one with no finite gate at or in front
+ * of it has h = 0, m = -inf and gradients of 0, wherever the padding ends.  (In the sequence-parallel form a rank whose
+ * segment begins so leaves exp(-m) out of the normaliser of those positions: their m is not known there.)
  * The first 256 bytes of a workspace hold a device status word that kernels set when they give up on
  * an internal wait; mlstm_read_status() copies it to the host (this one call synchronises the stream);
  * mlstm_forward_f16_static_status() does the same for the built-in array.

@@ -105,9 +105,9 @@ state_scan_kernel(const T16* __restrict__ U, const float* __restrict__ zU, const
             const int kb = reverse ? NB - 1 - (t0 + j) : t0 + j;
             const double b1 = bound[kb + 1], b0 = bound[kb];
             const double b1c = fmin(b1, lb), b0c = fmin(b0, lb);
-            // exp(A_end(k-1) - A_end(k)); 0 for the first block when there is no inbound carry (bound = +inf)
-            sd[j] = exp2f(static_cast<float>(b1c - b0c));
-            sc[j] = exp2f(static_cast<float>(b1c - b1));   // 1 unless the late carry raised the block's stabiliser
+            // exp(A_end(k-1) - A_end(k)); 0 while nothing is carried in (bound = +inf: also b1 then, in left padding)
+            sd[j] = b0c == static_cast<double>(INFINITY) ? 0.0f : exp2f(static_cast<float>(b1c - b0c));
+            sc[j] = b1c == b1 ? 1.0f : exp2f(static_cast<float>(b1c - b1));   // < 1: the late carry raised the block's stabiliser
         }
         __syncthreads();
         if (is_vec && !valid) continue;

@@ -451,18 +451,26 @@ mlstm_chunk_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             }
         };
         // FWDC with a late carry: the row's stabiliser and the inbound boundary are capped by the carried-in maximum, and m
-        // grows by what the cap took off.  Row weight of the carried state: FWDC, DQC exp(A_end(k-1) - A_t) (times scale,
-        // resp. scale / n_t); DKC, DVC exp(a_j - A_end(k)); 0 where nothing is carried in.
+        // grows by what the cap took off.  A row without a finite gate of its own (rel = -inf: left padding, gates.cu) has the
+        // carried-in maximum, if there is one, and then an m that is not known here (NaN: it takes no part in the normaliser).
+        auto capped = [&](float rel, double negA, double lb) {
+            return rel == -INFINITY && lb < static_cast<double>(INFINITY) ? lb : fmin(negA, lb);
+        };
+        // Row weight of the carried state: FWDC, DQC exp(A_end(k-1) - A_t) (times scale, resp. scale / n_t); DKC, DVC
+        // exp(a_j - A_end(k)); 0 where nothing is carried in, and for a position whose weights are all 0.
         auto combine = [&](const Item& it, const Raw& rr, Terms& tm) {
-            const double negA = static_cast<double>(rr.rel) + rr.ref;
-            const double lb = (IS_FWD && p.late_bound) ? rr.lb : static_cast<double>(INFINITY);
-            const double negA_c = IS_FWD ? fmin(negA, lb) : negA;
-            const double er_d = negA_c + static_cast<double>(p.er_add);
+            double negA = static_cast<double>(rr.rel) + rr.ref, bound = rr.b;
+            const bool none = it.tile >= NT || (rr.rel == -INFINITY && !(IS_FWD && p.late_bound));
+            if (IS_FWD && p.late_bound) {
+                const double negA_c = capped(rr.rel, negA, rr.lb);
+                tm.m = negA < negA_c ? NAN : tm.m + static_cast<float>((negA - negA_c) * 0.6931471805599453);
+                negA = negA_c;
+                bound = fmin(bound, rr.lb);
+            }
+            const double er_d = negA + static_cast<double>(p.er_add);
             tm.er[0] = static_cast<float>(er_d + rr.cr[0]);
             tm.er[1] = static_cast<float>(er_d + rr.cr[1]);
-            tm.state_w = it.tile >= NT ? 0.0f
-                                       : fast_exp2(ROWS_ARE_Q ? static_cast<float>(er_d - fmin(rr.b, lb)) : static_cast<float>(er_d + rr.b));
-            if (IS_FWD) tm.m += static_cast<float>((negA - negA_c) * 0.6931471805599453);
+            tm.state_w = none ? 0.0f : fast_exp2(static_cast<float>(ROWS_ARE_Q ? er_d - bound : er_d + bound));
         };
         // (plain loads, no __ldg: the first item's are not to move in front of grid_dep_wait)
         Raw raw{};
@@ -562,7 +570,7 @@ mlstm_chunk_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                     const int grow = tile * TILE + r;
                     double negA = static_cast<double>(p.row_rel[vec_base + grow]) +
                                   p.row_ref[static_cast<size_t>(bh) * (p.Spad / REF_BLOCK) + grow / REF_BLOCK];
-                    if (IS_FWD && p.late_bound) negA = fmin(negA, p.late_bound[bh]);
+                    if (IS_FWD && p.late_bound) negA = capped(p.row_rel[vec_base + grow], negA, p.late_bound[bh]);
                     er = static_cast<float>(negA + static_cast<double>(p.er_add) + column_ref(it, t));
                     w_own = column_term(it, t);
                     if (IS_DK) g_own = p.col_g[vec_base + st * TILE + cbase + lane];

@@ -90,6 +90,9 @@ static_assert(GATE_SEG_TOKENS == GATE_V * SCAN_THREADS && REF_BLOCK % GATE_V == 
 // A kernel forms exp2(col_rel[c] + float(row_rel[r] + row_ref[r / REF_BLOCK] + col_ref[c / REF_BLOCK])),
 // the bracket in double once per block of columns.  Padding (t >= S): ga_rel = -inf (a padded column
 // contributes exactly zero), gAn_rel = 0, references 0.  m may be null.
+// Left padding: positions in front of the slice's first finite input gate (i = -inf; A_t = -inf) see nothing.  Their
+// gAn_rel is -inf, so that every weight of the row is exactly 0 (m_t = -inf: h_t = 0), and An_ref of a block that begins
+// with such positions is that of its first finite A, 0 if it has none: no reference is infinite.
 // Chunkwise / sequence-parallel extras (all optional): carry_in[bh] = {F, A} at the end of the
 // preceding segment (natural-log units; absent = {0, -inf}); summary_out[bh] = {F, A} at the end of
 // this segment; An_bound[bh][0] = -A_in*log2e and An_bound[bh][k+1] = -A*log2e at the last position
@@ -210,6 +213,14 @@ __global__ void __launch_bounds__(SCAN_THREADS) gates_fwd_kernel(const T* __rest
         const double ra = (bm == -INFINITY) ? 0.0 : bm;
         const int lead = (threadIdx.x & 31) & ~(LANES_PER_REF - 1);      // lane that holds the block's first position
         double rA = __shfl_sync(0xffffffffu, A[0], lead);
+        if (__any_sync(0xffffffffu, rA == -INFINITY)) {      // a block that begins in front of the first finite gate
+            double first = INFINITY;                         // (A never decreases: its first finite value is its smallest)
+#pragma unroll
+            for (int j = 0; j < GATE_V; j++) first = A[j] > -INFINITY ? fmin(first, A[j]) : first;
+#pragma unroll
+            for (int o = LANES_PER_REF / 2; o > 0; o >>= 1) first = fmin(first, __shfl_xor_sync(0xffffffffu, first, o));
+            if (rA == -INFINITY) rA = first < INFINITY ? first : 0.0;
+        }
         if (base + GATE_V * (static_cast<int>(threadIdx.x) & ~(LANES_PER_REF - 1)) >= S) rA = 0.0;   // block of pure padding
         if (t0 < Spad && ga_rel) {
             float rel[GATE_V], w[GATE_V], An[GATE_V];
@@ -218,7 +229,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) gates_fwd_kernel(const T* __rest
                 const bool in = t0 + j < S;
                 rel[j] = in ? static_cast<float>((a[j] - ra) * LOG2E_D) : -INFINITY;
                 w[j] = exp2f(rel[j]);   // in (0, 1]; 0 in the padding
-                An[j] = in ? static_cast<float>((rA - A[j]) * LOG2E_D) : 0.0f;
+                An[j] = !in ? 0.0f : A[j] == -INFINITY ? -INFINITY : static_cast<float>((rA - A[j]) * LOG2E_D);
             }
             const size_t vi = static_cast<size_t>(bh) * Spad + t0;    // Spad and t0 are multiples of four
             *reinterpret_cast<float4*>(ga_rel + vi) = make_float4(rel[0], rel[1], rel[2], rel[3]);

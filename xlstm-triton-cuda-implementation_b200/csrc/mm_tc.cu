@@ -540,14 +540,19 @@ mlstm_tc_pass(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         const size_t vec_base = static_cast<size_t>(bh) * p.Spad;
         const size_t ref_base = static_cast<size_t>(bh) * (p.Spad / REF_BLOCK);
         // FWDC with a late carry: the row's stabiliser -A*log2e and the inbound block boundary are capped by the
-        // carried-in maximum, and m grows by what the cap took off
+        // carried-in maximum, and m grows by what the cap took off.  A row without a finite gate of its own (rel = -inf:
+        // left padding, gates.cu) has the carried-in maximum, if there is one, and then an m that is not known here (NaN:
+        // it takes no part in the normaliser).
+        const bool dark = raw.rel == -INFINITY;
         const double negA = static_cast<double>(raw.rel) + raw.ref;
-        const double negA_c = (MODE == FWDC) ? fmin(negA, raw.lb) : negA;
-        const float m_shift = (MODE == FWDC) ? static_cast<float>((negA - negA_c) * 0.6931471805599453) : 0.0f;
+        const double negA_c = (MODE != FWDC) ? negA : (dark && raw.lb < static_cast<double>(INFINITY)) ? raw.lb : fmin(negA, raw.lb);
+        const float m_shift = (MODE != FWDC) ? 0.0f
+                              : dark ? (p.late_bound ? NAN : 0.0f) : static_cast<float>((negA - negA_c) * 0.6931471805599453);
         const double er_d = negA_c + static_cast<double>(p.er_add);
         // log2 of the row weight of the state step: FWDC, DQC exp(A_end(k-1) - A_t) (times scale, resp. scale / n_t);
-        // DKC, DVC exp(a_j - A_end(k))
+        // DKC, DVC exp(a_j - A_end(k)); a position whose weights are all 0 has none (A_end(k) may be infinite there)
         const float er_state = !CHUNKED ? 0.0f
+                               : (dark && (MODE != FWDC || !p.late_bound)) ? -INFINITY
                                : ROWS_ARE_Q ? static_cast<float>(er_d - fmin(raw.b0, raw.lb)) : static_cast<float>(er_d + raw.b1);
         const float state_w = (MODE == DQC || MODE == DKC) ? fast_exp2(er_state) : 0.0f;   // for the epilogue's rank-1 term
         const float g_row = raw.g;

@@ -93,15 +93,16 @@ __global__ void __launch_bounds__(STEP_THREADS) step_kernel(const StepArgs p) {
             if (lane >= o) A = fmax(A, y);
         }
         const double A_end = __shfl_sync(0xffffffffu, A, T - 1);
+        // (weights of exactly 0 where there is nothing: no carried state, or an input gate of -inf, however A stands)
         if (lane < T) {
             s_a[lane] = a;
             s_A[lane] = A;
             s_m[lane] = static_cast<float>(F + A);
-            w_in[lane] = expf(static_cast<float>(A0 - A));
-            w_end[lane] = expf(static_cast<float>(a - A_end));
+            w_in[lane] = A0 == -INFINITY ? 0.0f : expf(static_cast<float>(A0 - A));
+            w_end[lane] = a == -INFINITY ? 0.0f : expf(static_cast<float>(a - A_end));
         }
         if (lane == T - 1) {
-            s_dec = expf(static_cast<float>(A0 - A_end));
+            s_dec = A0 == -INFINITY ? 0.0f : expf(static_cast<float>(A0 - A_end));
             if (blockIdx.x == 0) {
                 if (p.F_out) p.F_out[bh] = F;
                 if (p.A_out) p.A_out[bh] = A;
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(STEP_THREADS) step_kernel(const StepArgs p) {
         const float w0 = w_in[t] * p.scale;
         float b = w0 == 0.0f ? 0.0f : w0 * dot[t][TMAX];
         for (int j = 0; j <= t; j++) {
-            const float w = expf(static_cast<float>(s_a[j] - s_A[t])) * p.scale * dot[t][j];
+            const float w = s_a[j] == -INFINITY ? 0.0f : expf(static_cast<float>(s_a[j] - s_A[t])) * p.scale * dot[t][j];
             wt[t][j] = w;
             b += w;
         }
