@@ -79,7 +79,7 @@ template <int MODE, int D, int ABFMT, typename OutT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
 mlstm_chunk_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmYh,
                  const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmS,
-                 const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmO2, const PassParams p) {
+                 const __grid_constant__ CUtensorMap tmO, const PassParams p) {
     using C = CpCfg<D>;
     using InT = typename std::conditional<ABFMT == 1, __nv_bfloat16, __half>::type;
     constexpr bool ROWS_ARE_Q = (MODE == FWDC || MODE == DQC);
@@ -691,7 +691,7 @@ mlstm_chunk_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             [[maybe_unused]] const float rank1_coef = IS_DQ ? tm.state_w * tm.g : tm.state_w;
             // this warp's 32 rows x 32 columns (x the first of them) to global memory through its staging rows (16-byte pieces
             // swizzled over the bank groups, as the tensor map has it); rows past the end of the slice are not written
-            auto store_chunk = [&](const CUtensorMap* map, const uint32_t (&v)[32], int x) {
+            auto store_chunk = [&](const uint32_t (&v)[32], int x) {
                 constexpr int RB = sizeof(OutT) == 4 ? C::STAGE_ROW : 64;
                 constexpr int CPS = RB / static_cast<int>(sizeof(OutT));      // columns per store
 #pragma unroll
@@ -725,7 +725,7 @@ mlstm_chunk_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                     fence_async_smem();
                     __syncwarp();
                     if (lane == 0 && active) {
-                        tma_store_3d(map, stage, x + sub * CPS, row0, bh);
+                        tma_store_3d(&tmO, stage, x + sub * CPS, row0, bh);
                         bulk_commit();
                     }
                 }
@@ -757,7 +757,6 @@ mlstm_chunk_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                 if constexpr (IS_FWD) {
 #pragma unroll
                     for (int j = 0; j < 32; j++) av[j] = __float_as_uint(__uint_as_float(av[j]) * inv_n);
-                    if (p.out2) store_chunk(&tmO2, av, c0 + ch * 32);    // before the output gate
                 }
                 if (side_src) {
                     if (lane == 0) bulk_wait_read_all();
@@ -796,7 +795,7 @@ mlstm_chunk_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                     }
                     __syncwarp();
                 }
-                store_chunk(&tmO, av, c0 + ch * 32);
+                store_chunk(av, c0 + ch * 32);
             }
             // one partial per gate group: adding them up is left to the dF kernel, so that the groups need not meet here
             if ((IS_DQ || IS_DK) && p.dot_out && active)
@@ -823,18 +822,14 @@ mlstm_chunk_pair(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 template <int MODE, int D, int ABFMT, typename OutT>
 int launch_chunk_pair_one(const PassParams& p, int in_dtype, cudaStream_t st) {
     using C = CpCfg<D>;
-    CUtensorMap mx, myh, mz, ms, mo, mo2;
+    CUtensorMap mx, myh, mz, ms, mo;
     int rc;
     constexpr bool STATE_MN = (MODE == FWDC || MODE == DVC);
     constexpr int out_dtype = sizeof(OutT) == 4 ? MLSTM_DT_F32 : (ABFMT == 1 ? MLSTM_DT_BF16 : MLSTM_DT_F16);
     // staging rows of 128 bytes: the 128-byte swizzle of the operand maps; of 64 bytes: the output maps
-    auto out_map = [&](CUtensorMap* m, void* base) {
-        if (sizeof(OutT) == 4 && C::STAGE_ROW == 128) return tc_make_map(m, base, p.BH, p.S, D, out_dtype, false, 32);
-        return tc_make_map_out(m, base, p.BH, p.S, D, out_dtype, 32);
-    };
-    if ((rc = out_map(&mo, p.out)) != MLSTM_OK) return rc;
-    mo2 = mo;
-    if (p.out2 && (rc = out_map(&mo2, p.out2)) != MLSTM_OK) return rc;
+    rc = sizeof(OutT) == 4 && C::STAGE_ROW == 128 ? tc_make_map(&mo, p.out, p.BH, p.S, D, out_dtype, false, 32)
+                                                  : tc_make_map_out(&mo, p.out, p.BH, p.S, D, out_dtype, 32);
+    if (rc != MLSTM_OK) return rc;
     if ((rc = tc_make_map(&mx, p.X, p.BH, p.S, D, in_dtype, false, 128)) != MLSTM_OK) return rc;
     if ((rc = tc_make_map(&myh, p.Y, p.BH, p.S, D, in_dtype, false, 64)) != MLSTM_OK) return rc;
     if ((rc = tc_make_map(&mz, p.Z, p.BH, p.S, D, in_dtype, false, 128)) != MLSTM_OK) return rc;
@@ -867,17 +862,20 @@ int launch_chunk_pair_one(const PassParams& p, int in_dtype, cudaStream_t st) {
     if (sms < 2) return MLSTM_E_CUDA;
     // persistent pairs with equal shares; the grid does not have to be resident at once: CTAs only wait inside their pair
     const unsigned npairs = static_cast<unsigned>(total < sms / 2 ? total : sms / 2);
-    cudaError_t ce = launch_pdl(kern, dim3(2 * npairs), dim3(NTHREADS), C::SMEM_BYTES, st, mx, myh, mz, ms, mo, mo2, p);
+    cudaError_t ce = launch_pdl(kern, dim3(2 * npairs), dim3(NTHREADS), C::SMEM_BYTES, st, mx, myh, mz, ms, mo, p);
     if (ce != cudaSuccess) cudaGetLastError();
     return ce == cudaSuccess ? MLSTM_OK : note_cuda_error(ce, "launch of mlstm_chunk_pair");
 }
 
+// fp16: the output pass and DVC, which the chunkwise entry points use; DQC and DKC serve the bf16 route alone (mm_chunk_route)
 template <int MODE, int D>
 int launch_chunk_pair_fmt(const PassParams& p, int in_dtype, int out_dtype, cudaStream_t st) {
     if (in_dtype == MLSTM_DT_BF16) {
         if (out_dtype == in_dtype) return launch_chunk_pair_one<MODE, D, 1, __nv_bfloat16>(p, in_dtype, st);
         if constexpr (MODE == FWDC)
             if (out_dtype == MLSTM_DT_F32) return launch_chunk_pair_one<MODE, D, 1, float>(p, in_dtype, st);
+    } else if constexpr (MODE == DQC || MODE == DKC) {
+        return MLSTM_E_UNSUPPORTED;
     } else if (in_dtype == MLSTM_DT_F16) {
         if (out_dtype == in_dtype) return launch_chunk_pair_one<MODE, D, 0, __half>(p, in_dtype, st);
         if constexpr (MODE == FWDC)

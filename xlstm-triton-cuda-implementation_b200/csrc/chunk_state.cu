@@ -1,4 +1,5 @@
-// The states that the chunkwise form carries from block to block (16-bit inputs, head dimension 128 or 256):
+// The states that the chunkwise form carries from block to block (16-bit inputs, head dimension 128 or 256; the carried form
+// below for bf16 only):
 //     U_k = sum_j w_j x_j y_j^T,  w_j = exp2(col_rel_j + col_ref_j + bound)          (x_j, y_j the rows of block k)
 //     u_k = sum_j w_j g_j x_j                                                        (fp32; g_j = 1 in the forward)
 // forward   x = K, y = V, bound = -A_end(k):      the states of mlstm_scan.py:74-137 with the stabiliser known up front
@@ -439,10 +440,11 @@ int launch_states_one(const BlockStateArgs& p, int dtype, cudaStream_t st) {
 template <bool CARRY>
 int launch_states(const BlockStateArgs& p, int D, int dtype, cudaStream_t st) {
     if (!p.U || !p.vec || p.NB <= 0 || (dtype != MLSTM_DT_BF16 && dtype != MLSTM_DT_F16)) return MLSTM_E_ARG;
-    const bool bf = dtype == MLSTM_DT_BF16;
-    if (D == 128) return bf ? launch_states_one<128, 1, CARRY>(p, dtype, st) : launch_states_one<128, 0, CARRY>(p, dtype, st);
-    if (D == 256) return bf ? launch_states_one<256, 1, CARRY>(p, dtype, st) : launch_states_one<256, 0, CARRY>(p, dtype, st);
-    return MLSTM_E_UNSUPPORTED;
+    if (D != 128 && D != 256) return MLSTM_E_UNSUPPORTED;
+    if (dtype == MLSTM_DT_BF16)
+        return D == 128 ? launch_states_one<128, 1, CARRY>(p, dtype, st) : launch_states_one<256, 1, CARRY>(p, dtype, st);
+    if constexpr (CARRY) return MLSTM_E_UNSUPPORTED;      // (a carried sum may leave fp16's range)
+    else return D == 128 ? launch_states_one<128, 0, CARRY>(p, dtype, st) : launch_states_one<256, 0, CARRY>(p, dtype, st);
 }
 
 }  // namespace

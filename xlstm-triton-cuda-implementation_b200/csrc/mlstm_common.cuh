@@ -62,7 +62,6 @@ struct PassParams {
     const float* col_g;     // g per column (DK) or nullptr
     float er_add;           // constant term of er (FWD: log2(scale))
     void* out;           // [BH, S, D], element type chosen by the kernel template
-    void* out2;          // FWDC on CTA pairs: the result before the output gate (same type as out), or nullptr
     // FWD only
     const float* m;      // [BH, S] stabiliser, written by the gate pass
     float* b_out;        // [BH, S] row sums of the gated tile (the reference's B output) or nullptr
@@ -194,7 +193,7 @@ int launch_state_scan(const void* U, const float* zU, const double* An_bound, co
                       void* states16, float* zstate, float* S_end, float* z_end, int BH, int NB, int D, int dtype,
                       cudaStream_t st, const double* late_bound = nullptr, float* rec = nullptr, size_t rec_stride = 0,
                       const double* summary = nullptr, void* statesT16 = nullptr, int reverse = 0, int* zero_word = nullptr);
-// The parallel entry points' use of the chunkwise form (16-bit inputs, D = 128 or 256, long enough sequences): same
+// The parallel entry points' use of the chunkwise form (bf16 inputs, D = 128 or 256, long enough sequences): same
 // results, linear in S.  Nothing that the quadratic kernels keep in fp32 is rounded to 16 bits on the way: the carried
 // states, and what enters them, are held as two 16-bit halves (hi + mid).
 bool mm_chunk_route(int BH, int S, int D, int dtype, int flags);
