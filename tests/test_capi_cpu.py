@@ -68,21 +68,26 @@ def test_chunkwise_route_bounds_its_states(pkg):
 def test_workspace_falls_back_to_the_quadratic_form(pkg, monkeypatch):
     """Where the chunkwise form's states do not fit the memory the call asks for the quadratic kernels; nothing else does."""
     lib, L = pkg._lib, pkg._lib.lib()
-    query = lambda fl: L.mlstm_mm_fwd_workspace(1, 1, 8 << 20, 256, 2, fl)     # one slice: 8 GB of states
-    room = 1 << 30
 
     def alloc(nbytes, dev):
-        if nbytes > room:
+        if nbytes > 1 << 30:
             raise torch.OutOfMemoryError("no room")
         return nbytes
     monkeypatch.setattr(lib, "workspace", alloc)
-    assert lib.workspace_for(query, 0, "cuda") == (query(lib.F_FORCE_TC), lib.F_FORCE_TC)
-    room = 1 << 40
-    assert lib.workspace_for(query, 0, "cuda") == (query(0), 0)
-    room = 1 << 20
-    for q in (query, lambda fl: L.mlstm_mm_fwd_workspace(1, 8, 4096, 32, 0, fl)):   # (fp32, D = 32: no quadratic tensor-core form)
-        with pytest.raises(torch.OutOfMemoryError):
-            lib.workspace_for(q, 0, "cuda")
+
+    def get(S, D, query):       # as the entry points do
+        try:
+            return lib.workspace(query(0), "cuda"), 0
+        except torch.OutOfMemoryError:
+            return lib.workspace_or_less(query, 0, "cuda", S, D, 2)
+    query = lambda fl: L.mlstm_mm_fwd_workspace(1, 1, 8 << 20, 256, 2, fl)     # one slice: 8 GB of states
+    assert get(8 << 20, 256, query) == (query(lib.F_FORCE_TC), lib.F_FORCE_TC)
+    small = lambda fl: L.mlstm_mm_fwd_workspace(1, 8, 32768, 256, 2, fl)
+    assert get(32768, 256, small) == (small(0), 0)
+    with pytest.raises(torch.OutOfMemoryError):    # two passes: forcing the fused kernels would be an error
+        get(16384, 1024, lambda fl: L.mlstm_mm_bwd_workspace(1, 1, 16384, 1024, 2, 0, fl))
+    with pytest.raises(torch.OutOfMemoryError):    # the quadratic form does not fit either
+        get(65536, 256, lambda fl: L.mlstm_mm_bwd_workspace(4, 8, 65536, 256, 2, 0, fl))
 
 
 def test_bad_arguments_rejected_without_a_device(pkg):

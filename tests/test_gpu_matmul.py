@@ -422,6 +422,36 @@ def test_long_sequences_take_the_chunkwise_form(gc, BH, S, D, gated, pad):
             assert err(cut(a), r) < 1.25 * err(cut(a2), r), name
 
 
+def test_chunkwise_route_without_room_for_its_states(gc):
+    """With less memory than the block states need (the process' share is cut for the call) the parallel entry points run the
+    quadratic kernels: what MLSTM_F_FORCE_TC gives, bit for bit."""
+    B, NH, S, D = 1, 64, 2048, 256                       # states: 128 MB forward, 256 MB backward; scratch without: 1.5 and 69 MB
+    x = gc.make_inputs(B, NH, S, D, torch.bfloat16, f_mean=3.0, qkv_scale=D ** -0.5, seed=9)
+    d, dh = [x[n].cuda() for n in ("q", "k", "v", "f", "i")], x["dh"].cuda()
+
+    forward = lambda flags: gc.PKG.mlstm_matmul_forward(*d, flags=flags)
+    want = forward(gc._lib.F_FORCE_TC)
+    backward = lambda flags: gc.PKG.mlstm_matmul_backward(dh, *d, *want, flags=flags)
+    want_grads = backward(gc._lib.F_FORCE_TC)
+    assert not torch.equal(want[0], forward(0)[0])       # (another order of summation)
+    assert gc._lib.lib().mlstm_tc_supported(S, D, 2) == 1
+
+    def limited(fn, scratch):
+        """fn with room for its results and ``scratch`` bytes beside them"""
+        gc._lib._WS_CACHE.clear()
+        torch.cuda.empty_cache()
+        results = sum(t.numel() * t.element_size() for t in (want if fn is forward else want_grads))
+        room = torch.cuda.memory_reserved() + results + scratch
+        torch.cuda.set_per_process_memory_fraction(room / torch.cuda.get_device_properties(0).total_memory)
+        try:
+            return fn(0)
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+    for fn, scratch, ref in ((forward, 64 << 20, want), (backward, 160 << 20, want_grads)):
+        for a, r in zip(limited(fn, scratch), ref):
+            assert torch.equal(a, r)
+
+
 def test_chunkwise_route_in_slice_groups(gc):
     """More states than a set may hold (512 MB): the slices go in two groups of 33.  A slice's results do not depend on the
     slices beside it: both groups equal the same slices called on their own, in one group each."""

@@ -175,17 +175,13 @@ def workspace(nbytes: int, dev) -> torch.Tensor:
     return buf
 
 
-def workspace_for(query, flags: int, dev):
-    """(workspace, flags) of a call whose scratch size is ``query(flags)``.  Where the memory does not hold the scratch of the
-    form the library would choose (the chunkwise form of long sequences keeps block states) but does hold that of the
-    quadratic tensor-core kernels, the flags returned ask for those."""
-    nbytes = query(flags)
-    try:
-        return workspace(nbytes, dev), flags
-    except torch.OutOfMemoryError:
-        less = query(flags | F_FORCE_TC)
-        if not 0 < less < nbytes:
-            raise
+def workspace_or_less(query, flags: int, dev, S: int, D: int, dtype: int):
+    """(workspace, flags) for a call that has just run out of memory on its scratch of ``query(flags)`` bytes: where the form
+    the library would choose needs more (the chunkwise form of long sequences keeps block states) than the quadratic
+    tensor-core kernels, the flags returned ask for those; else the error goes on.  To be called while it is handled."""
+    less = query(flags | F_FORCE_TC)
+    if lib().mlstm_tc_supported(S, D, dtype) != 1 or not 0 < less < query(flags):
+        raise
     return workspace(less, dev), flags | F_FORCE_TC
 
 

@@ -20,6 +20,8 @@ fp32 dot products on the CUDA cores.  Setting the environment variable ``MLSTM_B
 
 Long bfloat16 sequences of many slices (D = 128 or 256, S >= 2048, B * NH * S >= 131072) are taken in blocks of 256 with
 a carried state (linear in S instead of quadratic; the state in fp32 and two 16-bit halves, so results are as accurate).
+The states take up to 512 MB of scratch forward and twice that backward (more for a single longer slice); where the memory
+does not hold them the call runs the quadratic kernels.
 
 Head dimensions above 256 (multiples of 256 up to 4096), 16-bit inputs, or float32 inputs with tf32 allowed:
 forward (float32 ``h``) and backward run on the tensor cores in two passes each (gated S x S matrices to scratch,
@@ -75,7 +77,10 @@ def mlstm_matmul_forward(q, k, v, f, i, h_dtype=torch.float32, flags=0):
     m = torch.empty((B, NH, S), device=dev, dtype=torch.float32)
     b = torch.empty((B, NH, S), device=dev, dtype=torch.float32)
     L = _lib.lib()
-    ws, flags = _lib.workspace_for(lambda fl: L.mlstm_mm_fwd_workspace(B, NH, S, D, dt, fl), flags, dev)
+    try:
+        ws = _lib.workspace(L.mlstm_mm_fwd_workspace(B, NH, S, D, dt, flags), dev)
+    except torch.OutOfMemoryError:
+        ws, flags = _lib.workspace_or_less(lambda fl: L.mlstm_mm_fwd_workspace(B, NH, S, D, dt, fl), flags, dev, S, D, dt)
     with torch.cuda.device(dev):
         rc = L.mlstm_mm_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), f.data_ptr(), i.data_ptr(), h.data_ptr(),
                             m.data_ptr(), b.data_ptr(), ws.data_ptr(), ws.numel(), B, NH, S, D, dt,
@@ -110,7 +115,10 @@ def _backward(dh, q, k, v, f, i, h, m, b, flags, o=None):
         _lib.require_cuda(q, o)
         do = torch.empty_like(o)
     query = L.mlstm_mm_bwd_workspace if o is None else L.mlstm_mm_bwd_ogate_workspace
-    ws, flags = _lib.workspace_for(lambda fl: query(B, NH, S, D, dt, hdt, fl), flags, dev)
+    try:
+        ws = _lib.workspace(query(B, NH, S, D, dt, hdt, flags), dev)
+    except torch.OutOfMemoryError:
+        ws, flags = _lib.workspace_or_less(lambda fl: query(B, NH, S, D, dt, hdt, fl), flags, dev, S, D, dt)
     with torch.cuda.device(dev):
         if o is not None:
             rc = L.mlstm_mm_bwd_ogate(dh.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), f.data_ptr(), i.data_ptr(),
