@@ -53,16 +53,22 @@ def test_workspace_sizes_and_support_matrix(pkg):
 
 
 def test_chunkwise_route_bounds_its_states(pkg):
-    """Long bf16 sequences behind the parallel entry points: block states of at most 512 MB per set (one set forward, two
-    backward) beside the row vectors that the quadratic kernels need as well, whatever the number of slices."""
+    """Long bf16 sequences behind the parallel entry points: beside the row vectors that the quadratic kernels need as well,
+    one set of block states forward and two backward, of at most 1 GB or of one wave of slices (148 CTAs, D / 128 per
+    slice, 4 D bytes per position), whatever the number of slices."""
     L, FORCE_TC, MB = pkg._lib.lib(), pkg._lib.F_FORCE_TC, 1 << 20
-    for B, NH, S, D in ((16, 8, 4096, 256), (32, 8, 131072, 256), (255, 16, 8192, 256), (64, 8, 65536, 128)):
+    for B, NH, S, D in ((16, 8, 4096, 256), (32, 8, 131072, 256), (255, 16, 8192, 256), (64, 8, 65536, 128), (1, 1, 1 << 20, 256)):
+        states = min(B * NH * S * 4 * D, max(1024 * MB, 148 * 128 * 4 * S))
         slack = 8 * MB + B * NH * S             # vector states, block boundaries, segments of the gate scan
         fwd = L.mlstm_mm_fwd_workspace(B, NH, S, D, 2, 0) - L.mlstm_mm_fwd_workspace(B, NH, S, D, 2, FORCE_TC)
-        assert 0 < fwd <= 512 * MB + slack, (B, NH, S, D, fwd)
+        assert 0 < fwd <= states + slack, (B, NH, S, D, fwd)
+        # ... and no fewer than keep the walk over the blocks at as many waves as all slices at once
+        one = -(-S // 256) * 4 * D * D
+        groups = -(-B * NH // max(1024 * MB // one, 148 * 128 // D))
+        assert fwd >= -(-B * NH // groups) * one, (B, NH, S, D, fwd)
         for query in (L.mlstm_mm_bwd_workspace, L.mlstm_mm_bwd_ogate_workspace):
             bwd = query(B, NH, S, D, 2, 0, 0) - query(B, NH, S, D, 2, 0, FORCE_TC)
-            assert 0 < bwd <= 1024 * MB + slack, (B, NH, S, D, bwd)
+            assert 0 < bwd <= 2 * states + slack, (B, NH, S, D, bwd)
 
 
 def test_workspace_falls_back_to_the_quadratic_form(pkg, monkeypatch):

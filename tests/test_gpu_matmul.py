@@ -453,9 +453,9 @@ def test_chunkwise_route_without_room_for_its_states(gc):
 
 
 def test_chunkwise_route_in_slice_groups(gc):
-    """More states than a set may hold (512 MB): the slices go in two groups of 33.  A slice's results do not depend on the
-    slices beside it: both groups equal the same slices called on their own, in one group each."""
-    BH, S, D, cut = 66, 8100, 256, 33
+    """More states than a set may hold (1 GB or 74 slices at D = 256): the slices go in two groups of 80.  A slice's results
+    do not depend on the slices beside it: both groups equal the same slices called on their own, in one group each."""
+    BH, S, D, cut = 160, 7100, 256, 80
     g = torch.Generator(device="cuda").manual_seed(5)
     rnd = lambda *shape: torch.randn(shape, device="cuda", generator=g)
     q, k, v, o = ((rnd(1, BH, S, D) * s).bfloat16() for s in (D ** -0.5, D ** -0.5, D ** -0.5, 1.0))

@@ -674,7 +674,8 @@ namespace mlstm {
 // states, B = 16, NH = 8, S = 4096, D = 256, forward + backward: 2.64 ms at 256, 2.91 at 512, 3.31 at 1024).
 constexpr int MM_CHUNK = 256;
 
-// Where the chunkwise form beats the quadratic kernels.  It needs slices (a CTA walks a slice's blocks, 5 us each) and length.
+// Where the chunkwise form beats the quadratic kernels.  It needs slices (a CTA walks a slice's blocks, 5 us each) and length:
+// with few slices the walk is long, but the quadratic cost, S times the number of positions, is longer still.
 // Measured bf16, us, quadratic -> chunkwise, forward | backward:
 //   D = 128   BH 32: S 2048 60 -> 70 | 203 -> 190, S 4096 148 -> 121 | 506 -> 338    BH 64: S 1024 44 -> 53 | 150 -> 156,
 //             S 2048 97 -> 88 | 343 -> 267    BH 128: S 1024 72 -> 74 | 250 -> 233, S 4096 596 -> 275 | 2135 -> 904
@@ -682,6 +683,11 @@ constexpr int MM_CHUNK = 256;
 //   D = 256   BH 32: S 2048 99 -> 101 | 284 -> 295, S 4096 221 -> 203 | 712 -> 569    BH 64: S 1024 78 -> 88 | 237 -> 261,
 //             S 2048 149 -> 148 | 496 -> 458    BH 128: S 1024 139 -> 149 | 456 -> 450, S 4096 986 -> 618 | 3128 -> 1791
 //             BH 16: S 4096 117 -> 140 | 375 -> 381, S 8192 375 -> 317 | 1182 -> 762
+// and along the line itself, S = 131072 / BH:
+//   D = 128   BH 1: 3695 -> 2220 | 12581 -> 4498, BH 2: 1876 -> 1156 | 6474 -> 2380, BH 4: 969 -> 631 | 3098 -> 1338,
+//             BH 8: 516 -> 354 | 1637 -> 788, BH 24: 223 -> 178 | 684 -> 434, BH 64: 123 -> 114 | 367 -> 291
+//   D = 256   BH 1: 5485 -> 2622 | 17035 -> 5373, BH 2: 2539 -> 1758 | 8995 -> 3166, BH 4: 1320 -> 937 | 4399 -> 1790,
+//             BH 8: 691 -> 438 | 2141 -> 1011, BH 24: 345 -> 245 | 944 -> 692, BH 64: 171 -> 169 | 511 -> 459
 // bf16 only: a state is a sum over positions, and fp16's range (65504) is too small for what the quadratic kernels add up
 // in fp32.  The forced paths keep the kernels they name.
 bool mm_chunk_route(int BH, int S, int D, int dtype, int flags) {
@@ -691,13 +697,20 @@ bool mm_chunk_route(int BH, int S, int D, int dtype, int flags) {
 }
 
 // Slices whose states are in the workspace at one time.  A state costs 4 D bytes per position of its slice (two 16-bit
-// matrices per block of 256), so slices go in groups of at most MM_STATE_BYTES of one set of states, of about the same size;
-// a slice that is longer than that goes alone.  One set forward, two backward (S_k and R_k).  At B = 16, NH = 8, S = 4096,
-// D = 256 a set is just one group.
-constexpr size_t MM_STATE_BYTES = size_t{512} << 20;
+// matrices per block of 256), so slices go in groups, of about the same size: as many as fit MM_STATE_BYTES of one set of
+// states, but no fewer than one wave of the states' kernel (D / 128 CTAs per slice on 148 SMs: 148 and 74 slices), because a
+// CTA walks its slice however few there are beside it, and smaller groups would walk one after the other.  A set then takes
+// at most MM_STATE_BYTES or 75 KB per position of the sequence, whatever the number of slices, and the groups walk in as many
+// waves as all slices at once would.  One set forward, two backward (S_k and R_k).
+// Measured, all slices at once -> two groups, us, forward | backward, both in turn (the runs of one side differ by 3 to 8 %):
+// 96 x 32768 at D = 256 3519 - 3746 -> 3417 - 3687 | 10620 - 11106 -> 10593 - 11123, 160 x 65536 at D = 128 5621 - 6108 ->
+// 5628 - 6074 | 17397 - 18643 -> 17748 - 18573.
+constexpr size_t MM_STATE_BYTES = size_t{1} << 30;
+constexpr int MM_WAVE_CTAS = 148;     // (a constant: the workspace query runs without a device)
 static int mm_chunk_group(int BH, int S, int D) {
     const size_t one = static_cast<size_t>((S + MM_CHUNK - 1) / MM_CHUNK) * D * D * 2 * 2;
-    const size_t most = one < MM_STATE_BYTES ? MM_STATE_BYTES / one : 1;
+    const size_t fit = MM_STATE_BYTES / one, wave = MM_WAVE_CTAS / (D / TILE);
+    const size_t most = fit > wave ? fit : wave;
     const int groups = static_cast<int>((BH + most - 1) / most);
     return (BH + groups - 1) / groups;
 }
