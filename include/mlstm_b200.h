@@ -68,9 +68,18 @@ int mlstm_tc_supported(int S, int D, int dtype);
  * mlstm_matmul_kernel (mlstm_matmul.py:37-101).
  *   q, k, v [B,NH,S,D], f, i [B,NH,S] of `dtype`; h [B,NH,S,D] of `h_dtype` (MLSTM_DT_F32 as the
  *   reference's Python path, or the input type); m, b [B,NH,S] fp32 (the reference's saved M, B).
- * D in {64, 128, 256}: one fused pass.  D = 512 .. 4096 in multiples of 256 with float32 h (16-bit inputs, or
- * float32 inputs with MLSTM_F_ALLOW_TF32): two tensor-core passes; the workspace then holds the gated matrices
- * of as many slices as fit 512 MB at once.  Everything else: the CUDA-core kernels.
+ * The form follows from shape, type and flags; the workspace query answers for the same ones:
+ *   D in {64, 128, 256} (float32 inputs: see MLSTM_F_ALLOW_TF32)   one fused pass, cost quadratic in S;
+ *   bf16, D = 128 or 256, S >= 2048 and B*NH*S >= 131072           blocks of 256 positions with a carried state, linear in S;
+ *        the workspace holds the states (4 D bytes per position) of as many slices as fit 1 GB, or of one wave of
+ *        slices where that is more (148 at D = 128, 74 at D = 256: 75 KB per position of the sequence).
+ *        MLSTM_F_FORCE_TC keeps the fused pass, which needs vectors per position only;
+ *   D = 512 .. 4096 in multiples of 256 with float32 h (16-bit inputs, or float32 inputs with MLSTM_F_ALLOW_TF32)
+ *        two tensor-core passes; the workspace holds the gated S x S matrices of as many slices as fit 512 MB;
+ *   everything else   the CUDA cores: up to D = 256 and S = 8192 in two stages, with the gated S x S matrices of as many
+ *        slices as fit 256 MB in the workspace, beyond that or with MLSTM_F_FORCE_SIMT or MLSTM_F_NO_SPLIT in one stage
+ *        without.  (Where the CUDA cores are the choice anyway, a query with MLSTM_F_FORCE_SIMT deliberately answers with the
+ *        size of the call without it, an upper bound; the call demands only what it uses.)
  */
 size_t mlstm_mm_fwd_workspace(int B, int NH, int S, int D, int dtype, int flags);
 int mlstm_mm_fwd(const void* q, const void* k, const void* v, const void* f, const void* i, void* h, float* m,
@@ -83,10 +92,13 @@ int mlstm_mm_fwd(const void* q, const void* k, const void* v, const void* f, con
  * mlstm_matmul_kernel_df (:319-333).
  *   dh, h of `h_dtype`; q, k, v, f, i and the outputs dq, dk, dv, df, di of `dtype`; m, b fp32 as
  *   written by mlstm_mm_fwd.  df[..., 0] is exactly 0 (mlstm_matmul.py:316, 392).
- * D in {64, 128, 256}: three fused passes (dQ, dK, dV).  D = 512 .. 4096 in multiples of 256 (16-bit inputs, or
- * float32 inputs with MLSTM_F_ALLOW_TF32): the normalised gated matrix and its gradient go to scratch (as many
- * slices at once as fit 512 MB), then dQ = dT K, dK = dT^T Q, dV = W^T dH as plain contractions: five
- * contractions in all.  Everything else: the CUDA-core kernels.
+ * The forms of the forward, by the same rules:
+ *   D in {64, 128, 256}: three fused passes (dQ, dK, dV);
+ *   long bf16 sequences: the same passes inside blocks of 256, with the states carried forward and back (two sets of
+ *        states, each bounded as in the forward);
+ *   D = 512 .. 4096 in multiples of 256 (any h_dtype): the normalised gated matrix and its gradient go to scratch (as
+ *        many slices at once as fit 512 MB), then dQ = dT K, dK = dT^T Q, dV = W^T dH as plain contractions, five in all;
+ *   CUDA cores in two stages: both matrices in scratch, 256 MB each.
  */
 size_t mlstm_mm_bwd_workspace(int B, int NH, int S, int D, int dtype, int h_dtype, int flags);
 int mlstm_mm_bwd(const void* dh, const void* q, const void* k, const void* v, const void* f, const void* i,

@@ -9,10 +9,13 @@
 // What bounds it: the state, read once and written once (B = 16, NH = 8, D = 128: 17 MB).  A CTA owns 32 columns (128
 // bytes of every row) of one slice's state, so that even a few sequences fill the chip, and holds its piece in registers:
 // all of its loads are in flight while the gates and the dot products q . k, q . z are taken, which every CTA of a slice
-// does for itself (T (T + 3) / 2 dots of length D).  A row of the state costs 2 T multiply-adds per element: 16 positions
-// stay near the memory's time.  More positions go through the tensor-core blocks of chunk.cu.
-// Measured (B = 16, NH = 8, D = 128, one bf16 position with the state in and out, call by call): 51 us, bound by the host's part
-// of the call, against 99 us through the five launches of a block of 256 positions.
+// does for itself (T (T + 3) / 2 dots of length D).  A row of the state costs 2 T multiply-adds per element, with their
+// operands from shared memory: with many sequences a call leaves the memory's time from a few positions on (see below).
+// Why up to 16 positions: as far as that it is faster than a block of chunk.cu at every number of sequences.  Kernel time, us,
+// bf16, state in and out, at T = 1 | 4 | 5 | 8 | 16 positions, and of the block's launches (which hardly depend on T):
+//   D = 128   BH 8: 6 | 8 | 10 | 10 | 19, block 25-27    BH 64: 6 | 8 | 10 | 12 | 21, 35-37    BH 512: 21 | 31 | 58 | 71 | 131, 165-170
+//   D = 256   BH 8: 6 | 8 | 10 | 12 | 21, block 33-35    BH 64: 10 | 16 | 21 | 25 | 45, 70      BH 256: 45 | 62 | 80 | 96 | 170, 250
+// A call takes at least 40 us, the host's part, against 77 us with the block's five launches.
 #include "mlstm_common.cuh"
 
 namespace mlstm {

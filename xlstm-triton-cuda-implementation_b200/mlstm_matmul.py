@@ -20,8 +20,8 @@ fp32 dot products on the CUDA cores.  Setting the environment variable ``MLSTM_B
 
 Long bfloat16 sequences of many slices (D = 128 or 256, S >= 2048, B * NH * S >= 131072) are taken in blocks of 256 with
 a carried state (linear in S instead of quadratic; the state in fp32 and two 16-bit halves, so results are as accurate).
-The states take up to 512 MB of scratch forward and twice that backward (more for a single longer slice); where the memory
-does not hold them the call runs the quadratic kernels.
+The states take up to 1 GB of scratch, or 75 KB per position of the sequence where that is more, and twice that in the
+backward; where the memory does not hold them the call runs the quadratic kernels.
 
 Head dimensions above 256 (multiples of 256 up to 4096), 16-bit inputs, or float32 inputs with tf32 allowed:
 forward (float32 ``h``) and backward run on the tensor cores in two passes each (gated S x S matrices to scratch,
