@@ -178,11 +178,12 @@ int sizing_flags(int S, int D, int dtype, int flags) {
 }
 // scratch of forward_impl behind the gate vectors: converted operands, or the two-stage form's matrices
 size_t fwd_extra_bytes(int BH, int S, int D, int dtype, int flags) {
-    return simt_two_stage(S, D, dtype, flags) ? simt_gemm_fwd_bytes(BH, S) : tf32_copy_bytes(BH, S, D, dtype, flags, 3);
+    const size_t vec = static_cast<size_t>(BH) * round_up(S, TILE) * sizeof(float);
+    return simt_two_stage(S, D, dtype, flags) ? al(simt_gemm_fwd_bytes(BH, S)) + al(vec) : tf32_copy_bytes(BH, S, D, dtype, flags, 3);
 }
 size_t simt_bwd_extra_bytes(int BH, int S, int D) {
     const size_t vec = static_cast<size_t>(BH) * round_up(S, TILE) * sizeof(float);
-    return 2 * al(simt_gemm_matrix_bytes(BH, S)) + 2 * al(vec * ((D + 63) / 64));
+    return 2 * al(simt_gemm_matrix_bytes(BH, S)) + 2 * al(vec * ((D + 63) / 64)) + al(vec);
 }
 
 int run_pass(int kind, int mode, const PassParams& p, int in_dt, int out_dt, cudaStream_t st) {
@@ -198,11 +199,13 @@ int forward_impl(const void* q, const void* k, const void* v, const void* f, con
     if (rc != MLSTM_OK) return rc;
     const int Spad = round_up(S, TILE);
     // (the gate pass also clears the status word and the passes' work-item counters)
+    const bool two_stage = extra && simt_two_stage(S, D, dtype, flags);
+    float* gAn_lo = two_stage ? reinterpret_cast<float*>(static_cast<uint8_t*>(extra) + al(simt_gemm_fwd_bytes(BH, S))) : nullptr;
     if ((rc = launch_gates_fwd(f, i, w.ga, w.gAn, w.a_ref, w.An_ref, m, BH, S, Spad, dtype, st, nullptr, nullptr, nullptr, 0, nullptr,
-                               w.gaw, w.status, STATUS_WORDS)) != MLSTM_OK)
+                               w.gaw, w.status, STATUS_WORDS, gAn_lo)) != MLSTM_OK)
         return rc;
-    if (extra && simt_two_stage(S, D, dtype, flags)) {
-        SimtGemmArgs a{S, Spad, BH, D, w.ga, w.gAn, w.a_ref, w.An_ref, m, b, static_cast<float*>(extra)};
+    if (two_stage) {
+        SimtGemmArgs a{S, Spad, BH, D, w.ga, w.gAn, w.gaw, gAn_lo, w.a_ref, w.An_ref, m, b, static_cast<float*>(extra)};
         return launch_simt_gemm_fwd(a, q, k, v, o, h, dtype, h_dtype, st);
     }
     const void* in[3] = {q, k, v};
@@ -412,18 +415,21 @@ static int mm_bwd_impl(const void* dh, const void* q, const void* k, const void*
     const int kind = pass_kind(S, D, dtype, flags, &rc);
     if (rc != MLSTM_OK) return rc;
 
+    // behind the vectors, two stages: the matrices, the row dots' partials, the rests of gAn
+    uint8_t* extra_base = static_cast<uint8_t*>(workspace) + w.bytes;
+    float* gAn_lo = two_stage ? reinterpret_cast<float*>(extra_base + extra - al(static_cast<size_t>(BH) * Spad * sizeof(float))) : nullptr;
     if ((rc = launch_gates_fwd(f, i, w.ga, w.gAn, w.a_ref, w.An_ref, nullptr, BH, S, Spad, dtype, st, nullptr, nullptr, nullptr, 0,
-                               nullptr, w.gaw, w.status, STATUS_WORDS)) != MLSTM_OK)
+                               nullptr, w.gaw, w.status, STATUS_WORDS, gAn_lo)) != MLSTM_OK)
         return rc;
-    if ((rc = launch_bwd_prep(h, dh, b, m, w.gAn, w.gB, w.gBw, w.g, w.dh16, o, d_o, BH, S, Spad, D, h_dtype, dtype, st)) != MLSTM_OK)
+    if ((rc = launch_bwd_prep(h, dh, b, m, w.gAn, w.gB, w.gBw, w.g, w.dh16, o, d_o, BH, S, Spad, D, h_dtype, dtype, st, gAn_lo)) != MLSTM_OK)
         return rc;
     const void* dhp = dh_es ? w.dh16 : dh;  // dh in the element type of q, k, v
     if (two_stage) {
-        uint8_t* base = static_cast<uint8_t*>(workspace) + w.bytes;
+        uint8_t* base = extra_base;
         const size_t mat = al(simt_gemm_matrix_bytes(BH, S)), vec = static_cast<size_t>(BH) * Spad * sizeof(float);
         const int nparts = (D + 63) / 64;
-        SimtGemmArgs a{S, Spad, BH, D, w.ga, w.gAn, w.a_ref, w.An_ref, nullptr, nullptr, reinterpret_cast<float*>(base)};
-        SimtGemmBwdArgs g{q, k, v, dhp, dq, dk, dv, w.gB, w.g, reinterpret_cast<float*>(base + mat), reinterpret_cast<float*>(base + 2 * mat),
+        SimtGemmArgs a{S, Spad, BH, D, w.ga, w.gAn, w.gaw, gAn_lo, w.a_ref, w.An_ref, nullptr, nullptr, reinterpret_cast<float*>(base)};
+        SimtGemmBwdArgs g{q, k, v, dhp, dq, dk, dv, w.gB, w.gBw, w.g, reinterpret_cast<float*>(base + mat), reinterpret_cast<float*>(base + 2 * mat),
                           reinterpret_cast<float*>(base + 2 * mat + al(vec * nparts)), static_cast<long long>(BH) * Spad};
         if ((rc = launch_simt_gemm_bwd(a, g, dtype, st)) != MLSTM_OK) return rc;
         return launch_df(f, g.dI, g.R, df, di, BH, S, Spad, dtype, st, nparts, g.dot_stride);

@@ -90,6 +90,9 @@ static_assert(GATE_SEG_TOKENS == GATE_V * SCAN_THREADS && REF_BLOCK % GATE_V == 
 // A kernel forms exp2(col_rel[c] + float(row_rel[r] + row_ref[r / REF_BLOCK] + col_ref[c / REF_BLOCK])),
 // the bracket in double once per block of columns.  Padding (t >= S): ga_rel = -inf (a padded column
 // contributes exactly zero), gAn_rel = 0, references 0.  m may be null.
+// LO: ga_w and gAn_lo receive what the rounding of ga_rel and gAn_rel to fp32 left out instead.  Both may be tens where the
+// exponent they make is of order 1; the fp32 form in two stages (simt_gemm.cu) adds the rests.  (A kernel of its own: as a
+// branch it cost every other form registers, 54 -> 64 with spills here and 80 -> 92 in bwd_prep_kernel.)
 // Left padding: positions in front of the slice's first finite input gate (i = -inf; A_t = -inf) see nothing.  Their
 // gAn_rel is -inf, so that every weight of the row is exactly 0 (m_t = -inf: h_t = 0), and An_ref of a block that begins
 // with such positions is that of its first finite A, 0 if it has none: no reference is infinite.
@@ -105,7 +108,7 @@ static_assert(GATE_SEG_TOKENS == GATE_V * SCAN_THREADS && REF_BLOCK % GATE_V == 
 // scans its segment with no carry, publishes the segment's {F, A} totals in coop_local, the grid meets, every block
 // folds the totals of the segments before it (carry_in and summary_out are then per SLICE) and shifts what it holds in
 // registers: F += F_in, a -= F_in, A = max(A - F_in, A_in).  One pass over f and i, one launch.
-template <typename T, bool COOP = false>
+template <typename T, bool COOP = false, bool LO = false>
 __global__ void __launch_bounds__(SCAN_THREADS) gates_fwd_kernel(const T* __restrict__ f, const T* __restrict__ i,
                                                                  float* __restrict__ ga_rel, float* __restrict__ gAn_rel,
                                                                  float* __restrict__ ga_w,
@@ -115,7 +118,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) gates_fwd_kernel(const T* __rest
                                                                  double* __restrict__ summary_out,
                                                                  double* __restrict__ An_bound, int chunk_len, int nseg,
                                                                  int seg_tokens, int* __restrict__ zero_words, int n_zero,
-                                                                 double* __restrict__ coop_local) {
+                                                                 double* __restrict__ coop_local, float* __restrict__ gAn_lo) {
     __shared__ double wsum[32];
     __shared__ double wmax[32];
     [[maybe_unused]] __shared__ double fold_in[2];
@@ -232,6 +235,15 @@ __global__ void __launch_bounds__(SCAN_THREADS) gates_fwd_kernel(const T* __rest
                 An[j] = !in ? 0.0f : A[j] == -INFINITY ? -INFINITY : static_cast<float>((rA - A[j]) * LOG2E_D);
             }
             const size_t vi = static_cast<size_t>(bh) * Spad + t0;    // Spad and t0 are multiples of four
+            if constexpr (LO) {
+                float lo[GATE_V];
+#pragma unroll
+                for (int j = 0; j < GATE_V; j++) {
+                    w[j] = rel[j] == -INFINITY ? 0.0f : static_cast<float>((a[j] - ra) * LOG2E_D - rel[j]);
+                    lo[j] = (t0 + j >= S || An[j] == -INFINITY) ? 0.0f : static_cast<float>((rA - A[j]) * LOG2E_D - An[j]);
+                }
+                *reinterpret_cast<float4*>(gAn_lo + vi) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+            }
             *reinterpret_cast<float4*>(ga_rel + vi) = make_float4(rel[0], rel[1], rel[2], rel[3]);
             if (ga_w) *reinterpret_cast<float4*>(ga_w + vi) = make_float4(w[0], w[1], w[2], w[3]);
             *reinterpret_cast<float4*>(gAn_rel + vi) = make_float4(An[0], An[1], An[2], An[3]);
@@ -287,6 +299,7 @@ __global__ void gates_fold_kernel(const double* __restrict__ local, const double
 // gate's backward costs no pass of its own.  Bound by HBM: dh, h, o in, dh_out, d_o out, 14 bytes per element (16-bit
 // inputs, fp32 h) where the gate's own kernel and this one moved 26.
 // Rows are read with 16-byte accesses.  Padding rows: gB_rel = -inf, g = 0.
+// LO (see gates_fwd_kernel): gB_w receives what the rounding of gB_rel left out, gAn_lo included.
 constexpr int PREP_ROWS = 4;   // positions per warp in bwd_prep_kernel
 
 // V consecutive values as one access
@@ -295,12 +308,12 @@ struct alignas(sizeof(T) * V) VecOf {
     T v[V];
 };
 
-template <typename HT, typename T16, bool GATED>
+template <typename HT, typename T16, bool GATED, bool LO>
 __global__ void bwd_prep_kernel(const HT* __restrict__ h, const HT* __restrict__ dh, const float* __restrict__ b,
                                 const float* __restrict__ m, const float* __restrict__ gAn_rel,
                                 float* __restrict__ gB_rel, float* __restrict__ gB_w, float* __restrict__ g,
                                 T16* __restrict__ dh_out, const T16* __restrict__ o, T16* __restrict__ d_o, int BH, int S,
-                                int Spad, int D, float log2_scale) {
+                                int Spad, int D, float log2_scale, const float* __restrict__ gAn_lo) {
     grid_dep_wait();
     grid_dep_launch();
     // A warp takes PREP_ROWS consecutive positions of one slice (Spad is a multiple of 128): all of their row
@@ -319,11 +332,13 @@ __global__ void bwd_prep_kernel(const HT* __restrict__ h, const HT* __restrict__
     const bool mine = lane < PREP_ROWS;
     const bool mine_valid = mine && tl < S;
     float bb = 0.0f, mm = 0.0f, ga = 0.0f;
+    [[maybe_unused]] float ga_lo = 0.0f;
     if (mine_valid) {
         const size_t idx = static_cast<size_t>(bh) * S + tl;
         bb = b[idx];
         mm = m[idx];
         ga = gAn_rel[first + lane];
+        if constexpr (LO) ga_lo = gAn_lo[first + lane];
     }
     float delta[PREP_ROWS];
 #pragma unroll
@@ -386,9 +401,10 @@ __global__ void bwd_prep_kernel(const HT* __restrict__ h, const HT* __restrict__
             const float db = (fabsf(bb) > em) ? sgn * (-my_delta / n) : 0.0f;
             const float gg = db * n;
             g[o] = isfinite(gg) ? gg : 0.0f;
-            const float rel = ga + (log2_scale - log2f(n));
+            const float c = log2_scale - log2f(n), rel = ga + c;
             gB_rel[o] = rel;
-            gB_w[o] = exp2f(rel);   // the same quantity as a factor, for the off-diagonal tiles
+            if constexpr (LO) gB_w[o] = rel == -INFINITY ? 0.0f : static_cast<float>(static_cast<double>(ga) + c - rel) + ga_lo;
+            else gB_w[o] = exp2f(rel);   // the same quantity as a factor, for the off-diagonal tiles
         }
     }
 }
@@ -663,13 +679,15 @@ int coop_capacity() {
 template <typename T>
 int gates_launch_typed(const void* f, const void* i, float* ga, float* gA, double* a_ref, double* An_ref, float* m, int BH,
                        int S, int Spad, cudaStream_t st, const double* carry_in, double* summary_out, double* An_bound,
-                       int chunk_len, double* scratch, float* ga_w, int* zero_words, int n_zero) {
+                       int chunk_len, double* scratch, float* ga_w, int* zero_words, int n_zero, float* gAn_lo) {
     const int nseg = scratch ? (Spad + GATE_SEG_TOKENS - 1) / GATE_SEG_TOKENS : 1;
     if (n_zero > SCAN_THREADS) return MLSTM_E_ARG;
+    if (gAn_lo && nseg > 1) return MLSTM_E_ARG;      // (the form that wants the rests passes no scratch)
     if (nseg <= 1) {
-        return launch_plain(gates_fwd_kernel<T, false>, dim3(BH), dim3(SCAN_THREADS), 0, st, (const T*)f, (const T*)i, ga, gA, ga_w, a_ref,
+        auto kern = gAn_lo ? gates_fwd_kernel<T, false, true> : gates_fwd_kernel<T, false>;
+        return launch_plain(kern, dim3(BH), dim3(SCAN_THREADS), 0, st, (const T*)f, (const T*)i, ga, gA, ga_w, a_ref,
                             An_ref, m, S, Spad, carry_in, summary_out, An_bound, chunk_len, 1, Spad, zero_words, n_zero,
-                            static_cast<double*>(nullptr)) == cudaSuccess
+                            static_cast<double*>(nullptr), gAn_lo) == cudaSuccess
                    ? MLSTM_OK : MLSTM_E_CUDA;
     }
     double* local = scratch;                                         // [BH * nseg][2]
@@ -686,7 +704,7 @@ int gates_launch_typed(const void* f, const void* i, float* ga, float* gA, doubl
         cfg.numAttrs = 1;
         cudaError_t ce = cudaLaunchKernelEx(&cfg, gates_fwd_kernel<T, true>, (const T*)f, (const T*)i, ga, gA, ga_w, a_ref, An_ref, m, S,
                                             Spad, carry_in, summary_out, An_bound, chunk_len, nseg, GATE_SEG_TOKENS, zero_words, n_zero,
-                                            local);
+                                            local, static_cast<float*>(nullptr));
         if (ce == cudaSuccess) return MLSTM_OK;
         cudaGetLastError();   // (not launched: take the three-launch path)
     }
@@ -697,14 +715,14 @@ int gates_launch_typed(const void* f, const void* i, float* ga, float* gA, doubl
     const double* nocd = nullptr;
     int* noi = nullptr;
     cudaError_t ce = launch_plain(gates_fwd_kernel<T, false>, dim3(BH * nseg), dim3(SCAN_THREADS), 0, st, (const T*)f, (const T*)i, nof, nof,
-                                  nof, nod, nod, nof, S, Spad, nocd, local, nod, 0, nseg, GATE_SEG_TOKENS, zero_words, n_zero, nod);
+                                  nof, nod, nod, nof, S, Spad, nocd, local, nod, 0, nseg, GATE_SEG_TOKENS, zero_words, n_zero, nod, nof);
     if (ce == cudaSuccess)
         ce = launch_plain(gates_fold_kernel, dim3((BH + 127) / 128), dim3(128), 0, st, (const double*)local, carry_in, seg_carry,
                         summary_out, BH, nseg);
     if (ce == cudaSuccess && (ga || m || An_bound))
         ce = launch_plain(gates_fwd_kernel<T, false>, dim3(BH * nseg), dim3(SCAN_THREADS), 0, st, (const T*)f, (const T*)i, ga, gA, ga_w,
                           a_ref, An_ref, m, S, Spad, (const double*)seg_carry, nod, An_bound, chunk_len, nseg, GATE_SEG_TOKENS, noi, 0,
-                          nod);
+                          nod, nof);
     return ce == cudaSuccess ? MLSTM_OK : MLSTM_E_CUDA;
 }
 }  // namespace
@@ -716,25 +734,25 @@ size_t gates_scratch_bytes(int BH, int Spad) {
 
 int launch_gates_fwd(const void* f, const void* i, float* ga, float* gA, double* a_ref, double* An_ref, float* m, int BH,
                      int S, int Spad, int dtype, cudaStream_t st, const double* carry_in, double* summary_out,
-                     double* An_bound, int chunk_len, double* scratch, float* ga_w, int* zero_words, int n_zero) {
+                     double* An_bound, int chunk_len, double* scratch, float* ga_w, int* zero_words, int n_zero, float* gAn_lo) {
     switch (dtype) {
         case MLSTM_DT_F32:
             return gates_launch_typed<float>(f, i, ga, gA, a_ref, An_ref, m, BH, S, Spad, st, carry_in, summary_out, An_bound,
-                                             chunk_len, scratch, ga_w, zero_words, n_zero);
+                                             chunk_len, scratch, ga_w, zero_words, n_zero, gAn_lo);
         case MLSTM_DT_F16:
             return gates_launch_typed<__half>(f, i, ga, gA, a_ref, An_ref, m, BH, S, Spad, st, carry_in, summary_out, An_bound,
-                                              chunk_len, scratch, ga_w, zero_words, n_zero);
+                                              chunk_len, scratch, ga_w, zero_words, n_zero, gAn_lo);
         case MLSTM_DT_BF16:
             return gates_launch_typed<__nv_bfloat16>(f, i, ga, gA, a_ref, An_ref, m, BH, S, Spad, st, carry_in, summary_out,
-                                                     An_bound, chunk_len, scratch, ga_w, zero_words, n_zero);
+                                                     An_bound, chunk_len, scratch, ga_w, zero_words, n_zero, gAn_lo);
     }
     return MLSTM_E_ARG;
 }
 
-template <typename HT, bool GATED>
+template <typename HT, bool GATED, bool LO>
 static int bwd_prep_dispatch(const void* h, const void* dh, const float* b, const float* m, const float* gA, float* gB,
                              float* gBw, float* g, void* dh_out, const void* o, void* d_o, int BH, int S, int Spad, int D,
-                             int dtype, cudaStream_t st) {
+                             int dtype, cudaStream_t st, const float* gAn_lo) {
     const long long warps = static_cast<long long>(BH) * Spad / PREP_ROWS;   // Spad is a multiple of 128
     const int threads = 256;
     const long long blocks = (warps * 32 + threads - 1) / threads;
@@ -742,14 +760,14 @@ static int bwd_prep_dispatch(const void* h, const void* dh, const float* b, cons
     const float log2_scale = -0.5f * log2f(static_cast<float>(D));
     const dim3 grid((unsigned)blocks), block(threads);
     if (dtype == MLSTM_DT_BF16)
-        launch_plain(bwd_prep_kernel<HT, __nv_bfloat16, GATED>, grid, block, 0, st, (const HT*)h, (const HT*)dh, b, m, gA, gB, gBw, g,
-                     (__nv_bfloat16*)dh_out, (const __nv_bfloat16*)o, (__nv_bfloat16*)d_o, BH, S, Spad, D, log2_scale);
+        launch_plain(bwd_prep_kernel<HT, __nv_bfloat16, GATED, LO>, grid, block, 0, st, (const HT*)h, (const HT*)dh, b, m, gA, gB, gBw, g,
+                     (__nv_bfloat16*)dh_out, (const __nv_bfloat16*)o, (__nv_bfloat16*)d_o, BH, S, Spad, D, log2_scale, gAn_lo);
     else if (dtype == MLSTM_DT_F16)
-        launch_plain(bwd_prep_kernel<HT, __half, GATED>, grid, block, 0, st, (const HT*)h, (const HT*)dh, b, m, gA, gB, gBw, g,
-                     (__half*)dh_out, (const __half*)o, (__half*)d_o, BH, S, Spad, D, log2_scale);
+        launch_plain(bwd_prep_kernel<HT, __half, GATED, LO>, grid, block, 0, st, (const HT*)h, (const HT*)dh, b, m, gA, gB, gBw, g,
+                     (__half*)dh_out, (const __half*)o, (__half*)d_o, BH, S, Spad, D, log2_scale, gAn_lo);
     else if constexpr (sizeof(HT) == 4)
-        launch_plain(bwd_prep_kernel<HT, float, GATED>, grid, block, 0, st, (const HT*)h, (const HT*)dh, b, m, gA, gB, gBw, g,
-                     (float*)dh_out, (const float*)o, (float*)d_o, BH, S, Spad, D, log2_scale);
+        launch_plain(bwd_prep_kernel<HT, float, GATED, LO>, grid, block, 0, st, (const HT*)h, (const HT*)dh, b, m, gA, gB, gBw, g,
+                     (float*)dh_out, (const float*)o, (float*)d_o, BH, S, Spad, D, log2_scale, gAn_lo);
     else
         return MLSTM_E_ARG;
     return cudaGetLastError() == cudaSuccess ? MLSTM_OK : MLSTM_E_CUDA;
@@ -757,16 +775,22 @@ static int bwd_prep_dispatch(const void* h, const void* dh, const float* b, cons
 
 int launch_bwd_prep(const void* h, const void* dh, const float* b, const float* m, const float* gA, float* gB, float* gBw,
                     float* g, void* dh_out, const void* o, void* d_o, int BH, int S, int Spad, int D, int h_dtype, int dtype,
-                    cudaStream_t st) {
-#define PREP(HT)                                                                                                          \
-    return o ? bwd_prep_dispatch<HT, true>(h, dh, b, m, gA, gB, gBw, g, dh_out, o, d_o, BH, S, Spad, D, dtype, st)         \
-             : bwd_prep_dispatch<HT, false>(h, dh, b, m, gA, gB, gBw, g, dh_out, nullptr, nullptr, BH, S, Spad, D, dtype, st)
+                    cudaStream_t st, const float* gAn_lo) {
+#define PREP_G(HT, LO)                                                                                                          \
+    return o ? bwd_prep_dispatch<HT, true, LO>(h, dh, b, m, gA, gB, gBw, g, dh_out, o, d_o, BH, S, Spad, D, dtype, st, gAn_lo) \
+             : bwd_prep_dispatch<HT, false, LO>(h, dh, b, m, gA, gB, gBw, g, dh_out, nullptr, nullptr, BH, S, Spad, D, dtype, st, gAn_lo)
+#define PREP(HT)                        \
+    do {                                \
+        if (gAn_lo) PREP_G(HT, true);   \
+        PREP_G(HT, false);              \
+    } while (0)
     switch (h_dtype) {
         case MLSTM_DT_F32: PREP(float);
         case MLSTM_DT_F16: PREP(__half);
         case MLSTM_DT_BF16: PREP(__nv_bfloat16);
     }
 #undef PREP
+#undef PREP_G
     return MLSTM_E_ARG;
 }
 

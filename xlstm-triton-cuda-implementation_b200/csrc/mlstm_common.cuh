@@ -165,7 +165,9 @@ int note_cuda_error(cudaError_t err, const char* where);
 int launch_gates_fwd(const void* f, const void* i, float* ga_rel, float* gAn_rel, double* a_ref, double* An_ref, float* m,
                      int BH, int S, int Spad, int dtype, cudaStream_t st, const double* carry_in = nullptr,
                      double* summary_out = nullptr, double* An_bound = nullptr, int chunk_len = 0,
-                     double* scratch = nullptr, float* ga_w = nullptr, int* zero_words = nullptr, int n_zero = 0);
+                     double* scratch = nullptr, float* ga_w = nullptr, int* zero_words = nullptr, int n_zero = 0,
+                     float* gAn_lo = nullptr);
+// gAn_lo: the rests of the vectors' rounding to gAn_lo and, in the place of the factors, to ga_w (gates.cu, LO)
 // zero_words / n_zero: device words the gate pass clears (the call's status block: status word and the work-item
 // counters of the passes that follow; STATUS_WORDS covers them all)
 constexpr int STATUS_WORDS = 64;
@@ -206,7 +208,7 @@ int mm_chunk_bwd(const void* dh, const void* q, const void* k, const void* v, co
                  int S, int D, int dtype, int h_dtype, cudaStream_t st);
 int launch_bwd_prep(const void* h, const void* dh, const float* b, const float* m, const float* gAn, float* gB,
                     float* gBw, float* g, void* dh_out, const void* o, void* d_o, int BH, int S, int Spad, int D, int h_dtype,
-                    int dtype, cudaStream_t st);
+                    int dtype, cudaStream_t st, const float* gAn_lo = nullptr);
 // dI, R: `nparts` partial vectors each, `part_stride` floats apart (see PassParams::dot_out).  scratch (optional,
 // gates_scratch_bytes(BH, Spad) bytes): long slices are then scanned in segments, one block each.
 int launch_df(const void* f, const float* dI, const float* R, void* df, void* di, int BH, int S, int Spad, int dtype,
@@ -218,7 +220,7 @@ int launch_pass_simt(int mode, const PassParams& p, int in_dtype, int out_dtype,
 // behind it); R, dI: [D / 64 rounded up][BH, Spad] partial row dots, dot_stride apart, for launch_df
 struct SimtGemmArgs {
     int S, Spad, BH, D;
-    const float *ga, *gAn;
+    const float *ga, *gAn, *ga_lo, *gAn_lo;     // _lo: with the rests of their rounding (gAn_lo of launch_gates_fwd)
     const double *a_ref, *An_ref;
     const float* m;
     float* b;
@@ -227,7 +229,7 @@ struct SimtGemmArgs {
 struct SimtGemmBwdArgs {
     const void *q, *k, *v, *dh;
     void *dq, *dk, *dv;
-    const float *gB, *g;
+    const float *gB, *gB_lo, *g;
     float *W1, *R, *dI;
     long long dot_stride;
 };

@@ -5,6 +5,10 @@
 // mm_simt.cu forms the gated tile again for every 64 output columns and every pass (at D = 256 forward and backward execute
 // 20 contractions); here each is executed once (2 and 5, the algorithmic count; the backward's two matrices serve three
 // results).  The sums are the same fp32 FMA sums.
+// One gated matrix for two results fixes which side's exponent is rounded first, which had moved dK, dV and dI 4 to 34 % away from
+// 64 bits against the one-stage passes at f ~ N(1, 1).  Row and column parts therefore carry the rests of their rounding (gAn_lo
+// of the gate pass): errors are 0.15 - 0.6 of the one-stage ones at f ~ N(1, 1), 0.15 - 0.93 at N(0, 1), 0.74 - 0.98 at N(3, 1)
+// (2-norm of h, dQ, dK, dV, dI; S 128 - 1664, D 32, 96, 256).  It costs 1 % (B = 1, NH = 4, S = 1024, D = 256: 104.3 -> 104.5 | 225.7 -> 228.7 us).
 //
 // What bounds it: the FMA units.  64 x 64 tiles on 128 threads of 8 x 4 results: per k step 32 FMA (8 cycles of an SM's
 // four schedulers for the CTA's four warps) against about 4 cycles of shared-memory reads; small tiles because a few heads
@@ -107,7 +111,7 @@ struct GateProblem {
 };
 struct GateArgs {
     GateProblem pr[2];
-    const float *row_rel, *col_rel;
+    const float *row_rel, *col_rel, *row_lo, *col_lo;
     const double *row_ref, *col_ref;
     float er_add;
     int S, Spad, D, Sp, bh0;
@@ -134,17 +138,28 @@ __global__ void __launch_bounds__(GTHREADS) simt_gate_kernel(const GateArgs p) {
     const double refs = p.row_ref[ref + rt] + p.col_ref[ref + ct] + static_cast<double>(p.er_add);
     const int col0 = ct * GT + tx * 4;
     const float4 ec4 = *reinterpret_cast<const float4*>(p.col_rel + vec + col0);
-    const float ec[4] = {ec4.x, ec4.y, ec4.z, ec4.w};
+    const float4 el4 = *reinterpret_cast<const float4*>(p.col_lo + vec + col0);
+    const float ec[4] = {ec4.x, ec4.y, ec4.z, ec4.w}, el[4] = {el4.x, el4.y, el4.z, el4.w};
     float* W = pr.W + static_cast<size_t>(slice) * p.Sp * p.Sp;
+    float row_rel[8], row_lo[8];      // (the loads of all rows in front of the first use)
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        row_rel[i] = p.row_rel[vec + rt * GT + ty * 8 + i];
+        row_lo[i] = p.row_lo[vec + rt * GT + ty * 8 + i];
+    }
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int row = rt * GT + ty * 8 + i;
-        const float er = static_cast<float>(static_cast<double>(p.row_rel[vec + row]) + refs);
+        // row and column part of the exponent as two floats each: they may be 60 and -60 where their sum is of order 1, and a
+        // rounding of the 60 would be a relative error of 2^-19 of the weight
+        const double er_d = static_cast<double>(row_rel[i]) + refs;
+        const float er = static_cast<float>(er_d);
+        const float er_lo = er == -INFINITY ? 0.0f : static_cast<float>(er_d - er) + row_lo[i];
         const float g = pr.g ? pr.g[vec + row] : 0.0f;
         float w[4], sum = 0.0f;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            w[j] = (acc[i][j] + g) * exp2f(ec[j] + er);
+            w[j] = (acc[i][j] + g) * exp2f((ec[j] + er) + (el[j] + er_lo));
             if (col0 + j > row || row >= p.S) w[j] = 0.0f;       // (a valid row's causal columns are valid)
             sum += w[j];
         }
@@ -257,7 +272,7 @@ int fwd_launch(const SimtGemmArgs& a, const void* q, const void* k, const void* 
         const int n = a.BH - bh0 < group ? a.BH - bh0 : group;
         GateArgs g{};
         g.pr[0] = GateProblem{q, k, nullptr, a.W0, a.W0 + static_cast<size_t>(group) * Sp * Sp};
-        g.row_rel = a.gAn; g.row_ref = a.An_ref; g.col_rel = a.ga; g.col_ref = a.a_ref;
+        g.row_rel = a.gAn; g.row_ref = a.An_ref; g.col_rel = a.ga; g.col_ref = a.a_ref; g.row_lo = a.gAn_lo; g.col_lo = a.ga_lo;
         g.er_add = -0.5f * log2f(static_cast<float>(a.D));
         g.S = a.S; g.Spad = a.Spad; g.D = a.D; g.Sp = Sp; g.bh0 = bh0;
         if (launch_plain(simt_gate_kernel<T>, dim3(NT * (NT + 1) / 2, n, 1), dim3(GTHREADS), 0, st, g) != cudaSuccess) return MLSTM_E_CUDA;
@@ -279,7 +294,7 @@ int bwd_launch(const SimtGemmArgs& a, const SimtGemmBwdArgs& b, cudaStream_t st)
         GateArgs g{};
         g.pr[0] = GateProblem{b.dh, b.v, b.g, a.W0, nullptr};      // dT
         g.pr[1] = GateProblem{b.q, b.k, nullptr, b.W1, nullptr};   // W / n
-        g.row_rel = b.gB; g.row_ref = a.An_ref; g.col_rel = a.ga; g.col_ref = a.a_ref;
+        g.row_rel = b.gB; g.row_ref = a.An_ref; g.col_rel = a.ga; g.col_ref = a.a_ref; g.row_lo = b.gB_lo; g.col_lo = a.ga_lo;
         g.S = a.S; g.Spad = a.Spad; g.D = a.D; g.Sp = Sp; g.bh0 = bh0;
         if (launch_plain(simt_gate_kernel<T>, dim3(NT * (NT + 1) / 2, n, 2), dim3(GTHREADS), 0, st, g) != cudaSuccess) return MLSTM_E_CUDA;
         ApplyArgs p{};
